@@ -67,32 +67,6 @@ k_sig_fill(const double *__restrict__ ll, long long n_rows, long long n_data,
     }
 }
 
-__global__ void __launch_bounds__(1024)
-k_scan_i32(const int *__restrict__ cnt, long long n, long long *__restrict__ off) {
-    __shared__ long long part[1024];
-    const long long per = (n + 1023) / 1024;
-    const long long lo = (long long)threadIdx.x * per, hi = min(n, lo + per);
-    long long s = 0;
-    for (long long i = lo; i < hi; ++i) s += cnt[i];
-    part[threadIdx.x] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        long long acc = 0;
-        for (int k = 0; k < 1024; ++k) {
-            long long v = part[k];
-            part[k] = acc;
-            acc += v;
-        }
-        off[n] = acc;
-    }
-    __syncthreads();
-    long long acc = part[threadIdx.x];
-    for (long long i = lo; i < hi; ++i) {
-        off[i] = acc;
-        acc += cnt[i];
-    }
-}
-
 // Bilinear footprint of detector pixel (x, y) under rotation (ac, as), the
 // geometry of slice_merge (kernels.cu:93-101).  Returns false off-detector.
 __device__ __forceinline__ bool footprint(int x, int y, int size, double ac, double as, int &ix,
@@ -213,7 +187,8 @@ extern "C" int rspi_posterior_pairs(const double *ll, long long n_rows, long lon
     const dim3 block(32, RY);
     const unsigned grid = (unsigned)((n_data + 31) / 32);
     k_sig_count<<<grid, block, 0, stream>>>(ll, n_rows, n_data, logz, p_min, cnt_part, cnt);
-    k_scan_i32<<<1, 1024, 0, stream>>>(cnt, n_data, off);
+    const int scan = rspi_scan_i32(cnt, n_data, off, stream);
+    if (scan != RSPI_OK) return scan;
     k_sig_fill<<<grid, block, 0, stream>>>(ll, n_rows, n_data, logz, p_min, cnt_part, off,
                                            capacity, pair_d, pair_r, pair_ll, err);
     RSPI_RETURN_LAUNCH();

@@ -275,43 +275,6 @@ extern "C" int rspi_ll_entry_rows(const int *ones, const int *multi, const long 
     RSPI_RETURN_LAUNCH();
 }
 
-namespace {
-// Exclusive scan of int32 row counts into int64 offsets with the total at [n].
-__global__ void __launch_bounds__(SCAN_THREADS)
-k_scan_rows(const int *__restrict__ rows, long long n, long long *__restrict__ off) {
-    __shared__ long long part[SCAN_THREADS];
-    const long long per = (n + SCAN_THREADS - 1) / SCAN_THREADS;
-    const long long lo = (long long)threadIdx.x * per;
-    const long long hi = min(n, lo + per);
-    long long s = 0;
-    for (long long i = lo; i < hi; ++i) s += rows[i];
-    part[threadIdx.x] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        long long acc = 0;
-        for (int k = 0; k < SCAN_THREADS; ++k) {
-            long long v = part[k];
-            part[k] = acc;
-            acc += v;
-        }
-        off[n] = acc;
-    }
-    __syncthreads();
-    long long acc = part[threadIdx.x];
-    for (long long i = lo; i < hi; ++i) {
-        off[i] = acc;
-        acc += rows[i];
-    }
-}
-}  // namespace
-
-extern "C" int rspi_scan_rows(const int *frame_rows, long long n_data, long long *row_off,
-                              cudaStream_t stream) {
-    if (n_data <= 0 || !frame_rows || !row_off) return RSPI_ERR_ARG;
-    k_scan_rows<<<1, SCAN_THREADS, 0, stream>>>(frame_rows, n_data, row_off);
-    RSPI_RETURN_LAUNCH();
-}
-
 extern "C" int rspi_ll_entry_fill(const int *ones, const int *multi, const long long *ones_accum,
                                   const long long *multi_accum, const int *place_ones,
                                   const int *place_multi, const int *count_multi,

@@ -184,3 +184,7 @@ static inline unsigned rspi_blocks(long long work, int threads, int cap_per_sm =
     if (b < 1) b = 1;
     return (unsigned)b;
 }
+
+// Exclusive scan of n int32 counts into off[0..n] (the total at [n]); one or
+// three launches (scan.cu).
+int rspi_scan_i32(const int *cnt, long long n, long long *off, cudaStream_t stream);

@@ -612,33 +612,6 @@ __global__ void k_cand_finalize(const long long *__restrict__ cand_off,
     }
 }
 
-// Scan of per-frame candidate counts (one CTA), with the total at [n].
-__global__ void __launch_bounds__(1024)
-k_scan_counts(const int *__restrict__ cnt, long long n, long long *__restrict__ off) {
-    __shared__ long long part[1024];
-    const long long per = (n + 1023) / 1024;
-    const long long lo = (long long)threadIdx.x * per, hi = min(n, lo + per);
-    long long s = 0;
-    for (long long i = lo; i < hi; ++i) s += cnt[i];
-    part[threadIdx.x] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        long long acc = 0;
-        for (int k = 0; k < 1024; ++k) {
-            long long v = part[k];
-            part[k] = acc;
-            acc += v;
-        }
-        off[n] = acc;
-    }
-    __syncthreads();
-    long long acc = part[threadIdx.x];
-    for (long long i = lo; i < hi; ++i) {
-        off[i] = acc;
-        acc += cnt[i];
-    }
-}
-
 }  // namespace
 
 extern "C" int rspi_ll16_entry_rows(const int *ones, const int *multi,
@@ -693,7 +666,8 @@ int candidates_launch(const float *ll, long long n_rows, long long n_x, long lon
     k_cand_count<<<grid, block, 0, stream>>>(ll, n_rows, n_x, stride, frame_of_col, max32,
                                              rmax32, frame_photons, row_off16, lmax, delta,
                                              cnt_part, cand_n, noncand, thr, cand_slot);
-    k_scan_counts<<<1, 1024, 0, stream>>>(cand_n, n_data, cand_off);
+    const int scan = rspi_scan_i32(cand_n, n_data, cand_off, stream);
+    if (scan != RSPI_OK) return scan;
     if (cand_slot)
         k_cand_compact<<<rspi_blocks(n_data * 32, 256), 256, 0, stream>>>(
             cand_slot, cnt_part, cand_off, n_data, capacity, cand_d, cand_r, err);
@@ -759,7 +733,8 @@ static int rescore_launch(const int *cand_d, const int *cand_r, const long long 
     const long long *total = cand_off + n_data;
     cudaMemsetAsync(row_cnt, 0, sizeof(int) * n_rows, stream);
     k_row_count<<<rspi_sm_count() * 8, 256, 0, stream>>>(cand_r, total, capacity, row_cnt);
-    k_scan_counts<<<1, 1024, 0, stream>>>(row_cnt, n_rows, row_cand_off);
+    const int scan = rspi_scan_i32(row_cnt, n_rows, row_cand_off, stream);
+    if (scan != RSPI_OK) return scan;
     cudaMemsetAsync(row_cnt, 0, sizeof(int) * n_rows, stream);
     k_row_scatter<<<rspi_sm_count() * 8, 256, 0, stream>>>(cand_r, total, capacity, row_cand_off,
                                                           row_cnt, row_cand);
@@ -897,7 +872,8 @@ extern "C" int rspi_screen_candidates_noalloc(const float *ll, long long n_rows,
     k_cand_count<<<grid, block, 0, stream>>>(ll, n_rows, n_data, n_data, nullptr, max32, rmax32,
                                              frame_photons, row_off16, lmax, delta, scratch,
                                              cand_n, noncand, thr, nullptr);
-    k_scan_counts<<<1, 1024, 0, stream>>>(cand_n, n_data, cand_off);
+    const int scan = rspi_scan_i32(cand_n, n_data, cand_off, stream);
+    if (scan != RSPI_OK) return scan;
     k_cand_fill<<<grid, block, 0, stream>>>(ll, n_rows, n_data, n_data, nullptr, nullptr, thr,
                                             rmax32, scratch, cand_off, capacity, cand_d, cand_r,
                                             err);
