@@ -203,9 +203,16 @@ k_histogram_map(const int *__restrict__ ones, const int *__restrict__ multi,
 __device__ __forceinline__ double2 fref_value(double qx, double qy, double qrad, double sx,
                                               double sy, double dia) {
     const double sval = xmul(xmul(PI, qrad), dia);
-    const double ff = xsub(sin(sval), xmul(sval, cos(sval))) / pow(sval, 3.);
+    double sn, cs;
+    sincos(sval, &sn, &cs);
+    // sval^3 to the last bit or so: the square and the cube with their
+    // rounding errors (pow took a third of the pattern search's set-up)
+    const double s2 = xmul(sval, sval), s3 = xmul(s2, sval);
+    const double cube = xadd(s3, fma(fma(sval, sval, -s2), sval, fma(s2, sval, -s3)));
+    const double ff = xsub(sn, xmul(sval, cs)) / cube;
     const double th = xmul(2. * PI, xadd(xmul(qx, sx), xmul(qy, sy)));
-    return make_double2(ff * cos(th), ff * sin(th));
+    sincos(th, &sn, &cs);
+    return make_double2(ff * cs, ff * sn);
 }
 
 struct PixelConsts {
@@ -377,85 +384,38 @@ constexpr int PT_CHUNK = 32;                       // FP32 terms per FP64 add
 constexpr double G_CHUNK = 32.01 * U32;            // gamma_32 (+ the FP64 adds)
 constexpr int NPART = 4;                           // partial sums per candidate
 static_assert(NPART == 4, "combine4 and sum_partials take four partial sums");
-constexpr int FIN_SPLIT = PT_THREADS / NPART;      // up to here: NPART threads each
-constexpr int FIN_CAP = NCAND;                     // beyond: a thread per finalist,
-                                                   // NPART sums, up to PT_CPT each
-
-__device__ __forceinline__ double block_max_d(double v, double *scratch) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int nw = (blockDim.x + 31) >> 5;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(RSPI_FULL_MASK, v, o));
-    __syncthreads();
-    if (lane == 0) scratch[wid] = v;
-    __syncthreads();
-    double m = -INFINITY;
-    for (int w = 0; w < nw; ++w) m = fmax(m, scratch[w]);
-    __syncthreads();
-    return m;
-}
-
-// Exclusive prefix of v in thread order, and the block total in *total.
-__device__ __forceinline__ int block_scan(int v, int *wsum, int *total) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int nw = (blockDim.x + 31) >> 5;
-    int x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(RSPI_FULL_MASK, x, o);
-        if (lane >= o) x += y;
-    }
-    __syncthreads();
-    if (lane == 31) wsum[wid] = x;
-    __syncthreads();
-    int before = 0, tot = 0;
-    for (int w = 0; w < nw; ++w) {
-        if (w < wid) before += wsum[w];
-        tot += wsum[w];
-    }
-    __syncthreads();
-    *total = tot;
-    return before + x - v;
-}
 
 // One FP32 screening term for a candidate held as hi + lo parts (xh, xl:
 // (real, imaginary)) against a populated state r = (re hi, im hi, re lo,
-// im lo), everything scaled by the pixel's power of two.  The real and
-// imaginary parts go through the packed FP32x2 adds (each lane rounded on
-// its own), and ab = (sum k l, sum k |l|) through one packed FMA.
-__device__ __forceinline__ void screen_term(float2 xh, float2 xl, const float4 r, float kj,
-                                            float &gmin, float2 &ab) {
-    const float2 z = __fadd2_rn(__fadd2_rn(xh, make_float2(r.x, r.y)),
-                                __fadd2_rn(xl, make_float2(r.z, r.w)));
+// im lo), everything scaled by the pixel's power of two: z = f_c + r into
+// `z`, |z|^2 returned.  The real and imaginary parts go through the packed
+// FP32x2 adds (each lane rounded on its own), and ab = (sum k l, sum k |l|)
+// through one packed FMA.
+__device__ __forceinline__ float screen_term(float2 xh, float2 xl, const float4 r, float kj,
+                                             float &gmin, float2 &ab, float2 &z) {
+    z = __fadd2_rn(__fadd2_rn(xh, make_float2(r.x, r.y)),
+                   __fadd2_rn(xl, make_float2(r.z, r.w)));
     const float g = fmaf(z.x, z.x, __fmul_rn(z.y, z.y));
     gmin = fminf(gmin, g);
     const float l = lg2_approx(g);
     ab = __ffma2_rn(make_float2(kj, kj), make_float2(l, fabsf(l)), ab);
+    return g;
 }
 
-// Per-pixel pattern search (maxLP.py:154-179, 304-340): one CTA per phaser
-// pixel (x mode), every thread PT_CPT candidates, the populated reference
-// states of the pixel in shared memory.
-//
-// SCREEN: each iteration first evaluates every candidate in FP32 (hi + lo
-// differences, lg2.approx, chunked sums) with a rigorous bound E_c on its
-// distance from the FP64 value; only the finalists, the candidates whose
-// upper end q32 + E reaches the best lower end max(q32 - E), are evaluated
-// in FP64 with the plain search's sums (four partial sums each, on four
-// threads or one).  The FP64 argmax is always a finalist and every other
-// candidate's FP64 value is strictly below it, so the chosen candidate is
-// the plain search's.  A candidate without a finite bound is a finalist.  A
-// pixel runs the plain FP64 iterations when it has more than one chunk of
-// populated states, counts >= 2^24, or is a ring pixel without photons.
-//
-// Bound, per term (u = 2^-24; A = |f_c|_inf + max_s |r_s|_inf, scaled):
-//   re, im from hi + lo parts: error <= 2u |re| + 6 u^2 A, so while
-//   |f_c + r|^2 >= max(2^-24 A^2, 2^-100) (checked through the minimum g):
-//   |ln g32 - ln g| <= 6.5 u, i.e. 9.5 u in log2;
-//   lg2: LG2_EA + LG2_ER |l|; chunk sums: gamma_32 sum k |l|.
-//   E_c = ln2 (K (LG2_EA + 9.5u) + (LG2_ER + g32)(1 + g32) sum k|l|) / n
-//         + 2^-40 (FP64 rounding of both evaluations).
-template <bool SCREEN>
+// Model pixel t's q (maxLP.py:79-85).
+__device__ __forceinline__ void pixel_consts_q(int t, int size, PixelConsts &pc) {
+    const double ds = (double)size, c0 = (double)(size / 2);
+    const int tx = t / size, ty = t - (t / size) * size;
+    pc.qx = ((double)tx - c0) / ds;
+    pc.qy = ((double)ty - c0) / ds;
+    pc.qrad = sqrt(xadd(xmul(pc.qx, pc.qx), xmul(pc.qy, pc.qy)));
+    if (pc.qrad == 0.) pc.qrad = 1.e-6;  // maxLP.py:85
+}
+
+// Plain per-pixel pattern search (maxLP.py:154-179, 304-340): one CTA per
+// phaser pixel (x mode), every thread PT_CPT candidates in FP64, the
+// populated reference states of the pixel in shared memory (in chunks of
+// POP_CAP).  `stats`, when given, counts its iterations in stats[1].
 __global__ void __launch_bounds__(PT_THREADS, 2)
 k_pattern(double2 *__restrict__ fconv, const int *__restrict__ pixels,
           const int *__restrict__ hist_row, long long n_pix, const int *__restrict__ hist,
@@ -464,9 +424,6 @@ k_pattern(double2 *__restrict__ fconv, const int *__restrict__ pixels,
           const double *__restrict__ rescale_ptr, int num_iter, double *__restrict__ rescale_out,
           unsigned long long *__restrict__ stats) {
     __shared__ double fr_re[POP_CAP], fr_im[POP_CAP], fk[POP_CAP];
-    __shared__ float4 r32[SCREEN ? POP_CAP : 1];
-    __shared__ float k32[SCREEN ? POP_CAP : 1];
-    __shared__ short fin[SCREEN ? FIN_CAP : 1];
     __shared__ double scratch[32];
     __shared__ int iscratch[32];
     __shared__ int wsum[32];
@@ -488,14 +445,7 @@ k_pattern(double2 *__restrict__ fconv, const int *__restrict__ pixels,
     }
 
     PixelConsts pc;
-    {
-        const double ds = (double)size, c0 = (double)(size / 2);
-        const int tx = t / size, ty = t - (t / size) * size;
-        pc.qx = ((double)tx - c0) / ds;
-        pc.qy = ((double)ty - c0) / ds;
-        pc.qrad = sqrt(xadd(xmul(pc.qx, pc.qx), xmul(pc.qy, pc.qy)));
-        if (pc.qrad == 0.) pc.qrad = 1.e-6;  // maxLP.py:85
-    }
+    pixel_consts_q(t, size, pc);
     // rbar, K total
     double ar = 0., ai = 0., ks = 0.;
     for (long long s = threadIdx.x; s < n_ref; s += blockDim.x) {
@@ -529,45 +479,9 @@ k_pattern(double2 *__restrict__ fconv, const int *__restrict__ pixels,
 
     const double kmean = pc.ksum / dn;
     const double rescale = ring ? 0. : rescale_ptr[mode];
-    // screen bound constants: the main pass's rho is the ring's mean rescale
-    // for every candidate, so its log is taken once per pixel; the bound
-    // multiplies by 1/dn (at most two ulps of q and e beyond the divisions,
-    // far inside its 2^-40 term)
-    const double inv_dn = 1. / dn;
-    const double lr_main = ring ? 0. : log(rescale);
     double2 f = fconv[t];
     double step = hypot(f.x, f.y) / 4.;
     const double shrink = 33. / 5.;  // sqrt(1089) / 5, maxLP.py:177
-
-    // FP32 copies of the populated states, scaled by 2^-sexp so that the
-    // largest of |f|_inf and max |r|_inf lies in [1/2, 1)
-    bool screen = false;
-    int sexp = 0;
-    double sc = 1., rinf_s = 0.;
-    if (SCREEN && one_chunk && !(ring && pc.ksum == 0.)) {
-        double rl = 0.;
-        int bad = 0;
-        for (int j = threadIdx.x; j < npop; j += blockDim.x) {
-            rl = fmax(rl, fmax(fabs(fr_re[j]), fabs(fr_im[j])));
-            bad |= !(fk[j] < 16777216.);
-        }
-        bad = __syncthreads_or(bad);
-        rl = block_max_d(rl, scratch);
-        const double top = fmax(rl, fmax(fabs(f.x), fabs(f.y)));
-        if (!bad && top > 0x1p-1000 && top < 0x1p1000) {
-            frexp(top, &sexp);
-            sc = ldexp(1., -sexp);
-            rinf_s = rl * sc;
-            for (int j = threadIdx.x; j < npop; j += blockDim.x) {
-                const double xr = fr_re[j] * sc, xi = fr_im[j] * sc;
-                const float hr = (float)xr, hi = (float)xi;
-                r32[j] = make_float4(hr, hi, (float)(xr - (double)hr), (float)(xi - (double)hi));
-                k32[j] = (float)fk[j];
-            }
-            __syncthreads();
-            screen = true;
-        }
-    }
 
     for (int it = 0; it < num_iter; ++it) {
         Cand cd[PT_CPT];
@@ -578,188 +492,47 @@ k_pattern(double2 *__restrict__ fconv, const int *__restrict__ pixels,
         }
         double best = -INFINITY;
         int bidx = 0x7fffffff;
-        bool searched = false;
-        if (SCREEN && screen) {
-            float2 xh[PT_CPT], xl[PT_CPT];
-            float gmin[PT_CPT];
-            double a64[PT_CPT], b64[PT_CPT];
+        // candidate by candidate (few live registers), each with its
+        // NPART partial sums: four independent logs in flight
+        double acc[PT_CPT][NPART];
+        if (one_chunk) {
 #pragma unroll
             for (int k = 0; k < PT_CPT; ++k) {
-                const double xs = cd[k].fr * sc, ys = cd[k].fi * sc;
-                xh[k] = make_float2((float)xs, (float)ys);
-                xl[k] = make_float2((float)(xs - (double)xh[k].x), (float)(ys - (double)xh[k].y));
-                gmin[k] = INFINITY;
-                a64[k] = 0.;
-                b64[k] = 0.;
+                double a4[NPART] = {0., 0., 0., 0.};
+                sum_partials(a4, cd[k], npop, fr_re, fr_im, fk);
+                acc[k][0] = combine4(a4[0], a4[1], a4[2], a4[3]);
             }
-            int j = 0;
-            for (; j + PT_CHUNK <= npop; j += PT_CHUNK) {
-                float2 ab[PT_CPT];
+        } else {
+            double part[PT_CPT][NPART];
 #pragma unroll
-                for (int k = 0; k < PT_CPT; ++k) ab[k] = make_float2(0.f, 0.f);
-#pragma unroll 2
-                for (int jj = 0; jj < PT_CHUNK; ++jj) {
-                    const float4 r = r32[j + jj];
-                    const float kj = k32[j + jj];
+            for (int k = 0; k < PT_CPT; ++k)
 #pragma unroll
-                    for (int k = 0; k < PT_CPT; ++k) screen_term(xh[k], xl[k], r, kj, gmin[k], ab[k]);
-                }
+                for (int p = 0; p < NPART; ++p) part[k][p] = 0.;
+            int s_next = 0;
+            do {
+                s_next = load_populated(s_next, hrow, n_ref, ref_params, pc, fr_re, fr_im, fk,
+                                        &npop, wsum);
 #pragma unroll
-                for (int k = 0; k < PT_CPT; ++k) {
-                    a64[k] += (double)ab[k].x;
-                    b64[k] += (double)ab[k].y;
-                }
-            }
-            {
-                float2 ab[PT_CPT];
-#pragma unroll
-                for (int k = 0; k < PT_CPT; ++k) ab[k] = make_float2(0.f, 0.f);
-                for (; j < npop; ++j) {
-                    const float4 r = r32[j];
-                    const float kj = k32[j];
-#pragma unroll
-                    for (int k = 0; k < PT_CPT; ++k) screen_term(xh[k], xl[k], r, kj, gmin[k], ab[k]);
-                }
-#pragma unroll
-                for (int k = 0; k < PT_CPT; ++k) {
-                    a64[k] += (double)ab[k].x;
-                    b64[k] += (double)ab[k].y;
-                }
-            }
-            // each candidate's interval [lo, hi] around its FP64 value
-            double lo[PT_CPT], up[PT_CPT];
-            const double ksum = pc.ksum, e2 = 2. * (double)sexp;
-#pragma unroll
-            for (int k = 0; k < PT_CPT; ++k) {
-                const int c = threadIdx.x + k * PT_THREADS;
-                lo[k] = -INFINITY;
-                up[k] = -INFINITY;
-                if (c >= NCAND) continue;
-                const double xs = cd[k].fr * sc, ys = cd[k].fi * sc;
-                const double amax = fmax(fabs(xs), fabs(ys)) + rinf_s;
-                const double thr = fmax(0x1p-24 * amax * amax, 0x1p-100);
-                const double rho = cd[k].rho, mwv = cd[k].mw;
-                bool safe = isfinite(a64[k]) && isfinite(b64[k]) && (double)gmin[k] >= thr &&
-                            amax >= 0x1p-38 && amax <= 0x1p60 && rho > 0. && rho < INFINITY &&
-                            isfinite(mwv);
-                if (safe) {
-                    const double lr = ring ? log(rho) : lr_main;
-                    const double q = (ksum * lr + LN2 * (a64[k] + e2 * ksum)) * inv_dn - rho * mwv;
-                    const double b2 = ksum * (LG2_EA + 9.5 * U32) +
-                                      (LG2_ER + G_CHUNK) * (1. + G_CHUNK) * b64[k];
-                    const double fm = 0x1p-40 * ((ksum * (fabs(lr) + LN2 * fabs(e2) + 1.) +
-                                                  LN2 * 1.01 * b64[k]) * inv_dn +
-                                                 fabs(rho * mwv));
-                    const double e = 1.001 * LN2 * b2 * inv_dn + fm;
-                    safe = isfinite(q) && isfinite(e);
-                    lo[k] = q - e;
-                    up[k] = q + e;
-                }
-                if (!safe) {
-                    lo[k] = -INFINITY;
-                    up[k] = INFINITY;
-                }
-            }
-            double tl = -INFINITY;
-#pragma unroll
-            for (int k = 0; k < PT_CPT; ++k) tl = fmax(tl, lo[k]);
-            tl = block_max_d(tl, scratch);
-            int mine = 0;
-#pragma unroll
-            for (int k = 0; k < PT_CPT; ++k) mine += (threadIdx.x + k * PT_THREADS < NCAND) && up[k] >= tl;
-            int nfin = 0;
-            int pos = block_scan(mine, wsum, &nfin);
-            // every candidate whose upper end reaches tl is a finalist (all
-            // of them when no candidate has a finite bound: tl = -inf)
-            {
-#pragma unroll
-                for (int k = 0; k < PT_CPT; ++k) {
-                    const int c = threadIdx.x + k * PT_THREADS;
-                    if (c < NCAND && up[k] >= tl) fin[pos++] = (short)c;
-                }
+                for (int k = 0; k < PT_CPT; ++k)
+                    sum_partials(part[k], cd[k], npop, fr_re, fr_im, fk);
                 __syncthreads();
-                if (nfin <= FIN_SPLIT) {
-                    // NPART consecutive threads per finalist, thread p summing
-                    // the states j = p mod NPART in order
-                    const int fi = threadIdx.x / NPART, part = threadIdx.x % NPART;
-                    double acc = 0.;
-                    Cand cc;
-                    if (fi < nfin) {
-                        cc = cand_at(fin[fi], f, step, pc, ring, kmean, rescale);
-                        for (int s = part; s < npop; s += NPART)
-                            acc = term64(acc, fk[s], cc, fr_re[s], fr_im[s]);
-                    }
-                    const double v1 = __shfl_down_sync(RSPI_FULL_MASK, acc, 1);
-                    const double v2 = __shfl_down_sync(RSPI_FULL_MASK, acc, 2);
-                    const double v3 = __shfl_down_sync(RSPI_FULL_MASK, acc, 3);
-                    if (fi < nfin && part == 0) {
-                        best = cand_q(combine4(acc, v1, v2, v3), dn, cc);
-                        bidx = fin[fi];
-                    }
-                } else {
-                    // one thread per finalist, its NPART sums in registers
-                    for (int i = threadIdx.x; i < nfin; i += PT_THREADS) {
-                        const int c = fin[i];
-                        const Cand cc = cand_at(c, f, step, pc, ring, kmean, rescale);
-                        double a4[NPART] = {0., 0., 0., 0.};
-                        sum_partials(a4, cc, npop, fr_re, fr_im, fk);
-                        const double q = cand_q(combine4(a4[0], a4[1], a4[2], a4[3]), dn, cc);
-                        if (argmax_better(q, c, best, bidx)) {
-                            best = q;
-                            bidx = c;
-                        }
-                    }
-                }
-                searched = true;
-                if (stats && threadIdx.x == 0) {
-                    atomicAdd(&stats[0], 1ull);
-                    atomicAdd(&stats[2], (unsigned long long)nfin);
-                }
+            } while (s_next < n_ref);
+#pragma unroll
+            for (int k = 0; k < PT_CPT; ++k)
+                acc[k][0] = combine4(part[k][0], part[k][1], part[k][2], part[k][3]);
+        }
+#pragma unroll
+        for (int k = 0; k < PT_CPT; ++k) {
+            const int c = threadIdx.x + k * PT_THREADS;
+            if (c >= NCAND) continue;
+            double q = cand_q(acc[k][0], dn, cd[k]);
+            if (ring && pc.ksum == 0.) q = NAN;  // 0 * log(0) in every frame
+            if (argmax_better(q, c, best, bidx)) {
+                best = q;
+                bidx = c;
             }
         }
-        if (!searched) {
-            // candidate by candidate (few live registers), each with its
-            // NPART partial sums: four independent logs in flight
-            double acc[PT_CPT][NPART];
-            if (one_chunk) {
-#pragma unroll
-                for (int k = 0; k < PT_CPT; ++k) {
-                    double a4[NPART] = {0., 0., 0., 0.};
-                    sum_partials(a4, cd[k], npop, fr_re, fr_im, fk);
-                    acc[k][0] = combine4(a4[0], a4[1], a4[2], a4[3]);
-                }
-            } else {
-                double part[PT_CPT][NPART];
-#pragma unroll
-                for (int k = 0; k < PT_CPT; ++k)
-#pragma unroll
-                    for (int p = 0; p < NPART; ++p) part[k][p] = 0.;
-                int s_next = 0;
-                do {
-                    s_next = load_populated(s_next, hrow, n_ref, ref_params, pc, fr_re, fr_im, fk,
-                                            &npop, wsum);
-#pragma unroll
-                    for (int k = 0; k < PT_CPT; ++k)
-                        sum_partials(part[k], cd[k], npop, fr_re, fr_im, fk);
-                    __syncthreads();
-                } while (s_next < n_ref);
-#pragma unroll
-                for (int k = 0; k < PT_CPT; ++k)
-                    acc[k][0] = combine4(part[k][0], part[k][1], part[k][2], part[k][3]);
-            }
-#pragma unroll
-            for (int k = 0; k < PT_CPT; ++k) {
-                const int c = threadIdx.x + k * PT_THREADS;
-                if (c >= NCAND) continue;
-                double q = cand_q(acc[k][0], dn, cd[k]);
-                if (ring && pc.ksum == 0.) q = NAN;  // 0 * log(0) in every frame
-                if (argmax_better(q, c, best, bidx)) {
-                    best = q;
-                    bidx = c;
-                }
-            }
-            if (SCREEN && stats && threadIdx.x == 0) atomicAdd(&stats[1], 1ull);
-        }
+        if (stats && threadIdx.x == 0) atomicAdd(&stats[1], 1ull);
         block_argmax(best, bidx, scratch, iscratch);
         const double px = -8. + 0.5 * (bidx / 33), py = -8. + 0.5 * (bidx % 33);
         const double2 fnew = make_double2(xadd(f.x, xmul(px, step)), xadd(f.y, xmul(py, step)));
@@ -769,6 +542,714 @@ k_pattern(double2 *__restrict__ fconv, const int *__restrict__ pixels,
         step = step_new;
     }
     if (threadIdx.x == 0) {
+        fconv[t] = f;
+        if (rescale_out) {   // maxLP.py:328, with the candidates' explicit roundings
+            const double er = xadd(f.x, pc.ar), ei = xadd(f.y, pc.ai);
+            rescale_out[mode * n_pix + ip] = kmean / fma(er, er, fma(ei, ei, pc.var));
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Screened pattern search: the plain search's candidate in every iteration,
+// from FP32 bounds.
+//
+// One CTA of four warps per phaser pixel (x mode), many CTAs on an SM.  The
+// plain search evaluates 1,089 candidates x populated states; here the 33 x
+// 33 pattern is cut into 11 x 11 cells of 3 x 3 candidates and an iteration
+// runs:
+//  1. a cell per thread: its centre c0 evaluated in FP32 (value q0, bound
+//     E0 on its distance from the FP64 value), with G = sum k z / |z|^2 and
+//     H = sum k / |z|^2 over the populated states, z = f_c0 + r.  Since
+//     log|1 + w|^2 <= 2 Re w + |w|^2 for every complex w, the log term of a
+//     neighbour c0 + d is at most the centre's plus 2 d.G + |d|^2 H, and the
+//     rest of its value (the rescaled mean intensity; the ring pass's
+//     rescale) is a known function of d: an upper bound U(d) for the cell's
+//     nine candidates.  tl = max(q0 - E0) is a lower bound on the best
+//     value; candidates with U < tl are out.
+//  2. the survivors in FP32, four threads each, with the same bound E; tl
+//     rises to their best q - E.
+//  3. the finalists, q + E >= tl, in FP64 with the plain search's sums (four
+//     partial sums, a thread each); the first index of the largest wins.
+// Where every candidate lies within |z| / 8 of f for every populated state
+// (a small step, or a model value far below the reference's: most pixels at
+// high q, where FP32 cannot tell the candidates apart), 1 and 2 give way to
+//  0. the expansion of the log terms around f to order 8, sum k log|z + d|^2
+//     = sum k log|z|^2 + 2 Re sum_m (-1)^(m+1) d^m (sum k / z^m) / m, in
+//     values relative to f's (so FP32 tells the candidates apart): a
+//     polynomial per candidate instead of a log per (candidate, state), with
+//     the remainder, the rounding and the plain search's own as its bound.
+// A single finalist is the choice without its FP64 value.
+// The FP64 argmax survives every test and every other finalist is compared
+// with it in FP64, so the choice is the plain search's, bit for bit.  A
+// candidate without a finite bound (out of the FP32 range, a term too close
+// to zero) always survives.  A pixel runs the FP64 search when a count
+// reaches 2^24 or its values leave the FP32 range; a ring pixel without
+// photons takes candidate 0, as NaN values do, and so does a zero step.
+//
+// Bound E, per term (u = 2^-24; A = |f_c|_inf + max_s |r_s|_inf, scaled):
+//   re, im from hi + lo parts: error <= 2u |re| + 6 u^2 A, so while
+//   |f_c + r|^2 >= max(2^-24 A^2, 2^-100) (checked through the minimum g):
+//   |ln g32 - ln g| <= 6.5 u, i.e. 9.5 u in log2;
+//   lg2: LG2_EA + LG2_ER |l|; chunk sums: gamma_32 sum k |l|.
+//   E = ln2 (K (LG2_EA + 9.5u) + (LG2_ER + g32)(1 + g32) sum k|l|) / n
+//       + 2^-40 (FP64 rounding of both evaluations).
+// U adds to q0 + E0: 2^-13 (2 |d| sqrt(K H) + |d|^2 H) / n for the FP32 sums
+// G and H of up to 1,024 terms (2^-14 of sum k/|z| <= sqrt(K H), and of H),
+// 2^-18 of the quadratic's own terms for its FP32 arithmetic and for the
+// candidates' rounded positions (d >= 2^-30 A is required), and the FP64
+// rounding of any candidate of the cell, 2^-30 of the value's terms.
+//
+// What bounds it is instruction issue and, for few pixels, the chain of an
+// iteration: ~14 instructions per (cell, state) for 121 cells instead of ~9
+// per (candidate, state) for 1,089, and 4 barriers of four warps instead of
+// 11 of twelve.  Measured, both passes together, against one CTA of 384
+// threads per pixel evaluating every candidate in FP32: 185^2, 20,000 frames
+// of 2,000 photons 3.4 ms (12.0), the same detector with three models and
+// 4,001 frames of uneven counts 6.5 ms (19.1), 101^2 with 1,000 frames 0.75
+// ms (2.06), 41^2 with 60 frames 0.30 ms (0.42); 1.3 finalists an iteration
+// instead of 43 at the first.
+constexpr int PS_THREADS = 128;
+constexpr int PS_CTAS = 6;                         // CTAs per SM (80 registers; 5 and 8 measured within 3%)
+constexpr int PS_WARPS = PS_THREADS / 32;
+constexpr int PS_VIRT = PT_THREADS / PS_THREADS;   // the plain search's threads per thread
+constexpr int PS_CELLS = 121;
+constexpr int PS_ORDER = 8;                        // of the expansion
+static_assert(PS_CELLS <= PS_THREADS, "a cell per thread");
+static_assert(PT_THREADS % PS_THREADS == 0, "set-up sums follow the plain search's threads");
+
+__device__ __forceinline__ float rcp_approx(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// block_sum of PT_THREADS virtual threads (virtual thread i + PS_THREADS v is
+// v[..][v] of thread i) for N sums at once: the same warps, the same order,
+// the same bits; every thread gets the sums.
+template <int N>
+__device__ __forceinline__ void virtual_block_sums(double (&v)[N][PS_VIRT], double (&out)[N],
+                                                   double (*scratch)[PS_VIRT * PS_WARPS]) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+#pragma unroll
+        for (int i = 0; i < PS_VIRT; ++i) {
+            const double w = warp_sum(v[k][i]);
+            if (lane == 0) scratch[k][wid + i * PS_WARPS] = w;
+        }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < N; ++k) out[k] = warp_sum(lane < PS_VIRT * PS_WARPS ? scratch[k][lane] : 0.);
+}
+
+// A pixel's constants for the FP32 bounds.
+struct ScreenConsts {
+    double ksum, inv_dn, lr_main, sc, rinf, e2;
+    bool ring;
+};
+
+// Value q and bound e of a candidate from its FP32 sums a = sum k l, b =
+// sum k |l| and the least |z|^2; fm is the FP64-rounding part's scale (the
+// bound holds 2^-40 of it).  False: no finite bound.
+__device__ __forceinline__ bool cand_bound(const Cand &cd, double a, double b, float gmin,
+                                           const ScreenConsts &k, double &q, double &e,
+                                           double &fm, double &amax) {
+    amax = fmax(fabs(cd.fr), fabs(cd.fi)) * k.sc + k.rinf;
+    const double thr = fmax(0x1p-24 * amax * amax, 0x1p-100);
+    if (!(isfinite(a) && isfinite(b) && (double)gmin >= thr && amax >= 0x1p-38 &&
+          amax <= 0x1p60 && cd.rho > 0. && cd.rho < INFINITY && isfinite(cd.mw)))
+        return false;
+    const double lr = k.ring ? log(cd.rho) : k.lr_main;
+    q = (k.ksum * lr + LN2 * (a + k.e2 * k.ksum)) * k.inv_dn - cd.rho * cd.mw;
+    const double b2 = k.ksum * (LG2_EA + 9.5 * U32) + (LG2_ER + G_CHUNK) * (1. + G_CHUNK) * b;
+    fm = (k.ksum * (fabs(lr) + LN2 * fabs(k.e2) + 1.) + LN2 * 1.01 * b) * k.inv_dn +
+         fabs(cd.rho * cd.mw);
+    e = 1.001 * LN2 * b2 * k.inv_dn + 0x1p-40 * fm;
+    return isfinite(q) && isfinite(e);
+}
+
+// Appends `count` entries per thread to a shared list of the CTA: the
+// thread's first position.
+__device__ __forceinline__ int list_push(int count, int *total) {
+    const int lane = threadIdx.x & 31;
+    int x = count;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(RSPI_FULL_MASK, x, o);
+        if (lane >= o) x += y;
+    }
+    int base = 0;
+    if (lane == 31 && x > 0) base = atomicAdd(total, x);
+    return __shfl_sync(RSPI_FULL_MASK, base, 31) + x - count;
+}
+
+// Appends `v` of the threads with `hit` to a shared list of the CTA.
+__device__ __forceinline__ void list_add(bool hit, short v, short *list, int *total) {
+    const unsigned bal = __ballot_sync(RSPI_FULL_MASK, hit);
+    if (bal == 0) return;
+    const int lane = threadIdx.x & 31;
+    int base = 0;
+    if (lane == 0) base = atomicAdd(total, __popc(bal));
+    base = __shfl_sync(RSPI_FULL_MASK, base, 0);
+    if (hit) list[base + __popc(bal & ((1u << lane) - 1u))] = v;
+}
+
+// The plain FP64 evaluation of n listed candidates, a thread each (no list:
+// every candidate, of a pixel out of the screen's range): this thread's best
+// value and its index.
+__device__ __noinline__ void plain_candidates(const short *list, int n, double2 f, double step, const PixelConsts &pc,
+                                              bool ring, double kmean, double rescale, double dn,
+                                              int npop, const double *re, const double *im,
+                                              const short *idx, const int *__restrict__ hrow,
+                                              double &best, int &bidx) {
+    for (int i = threadIdx.x; i < n; i += PS_THREADS) {
+        const int c = list ? list[i] : i;
+        const Cand cd = cand_at(c, f, step, pc, ring, kmean, rescale);
+        double a[NPART] = {0., 0., 0., 0.};
+        for (int j0 = 0; j0 < npop; j0 += NPART)
+#pragma unroll
+            for (int p = 0; p < NPART; ++p)
+                if (j0 + p < npop)
+                    a[p] = term64(a[p], (double)hrow[idx[j0 + p]], cd, re[j0 + p], im[j0 + p]);
+        const double q = cand_q(combine4(a[0], a[1], a[2], a[3]), dn, cd);
+        if (argmax_better(q, c, best, bidx)) {
+            best = q;
+            bidx = c;
+        }
+    }
+}
+
+__host__ __device__ constexpr int ps_state_bytes() { return 16 + 8 + 8 + 4 + 2; }
+
+__global__ void __launch_bounds__(PS_THREADS, PS_CTAS)
+k_pattern_screen(double2 *__restrict__ fconv, const int *__restrict__ pixels,
+                 const int *__restrict__ hist_row, long long n_pix, const int *__restrict__ hist,
+                 int n_ref, int cap, const int *__restrict__ nstate, long long n_modes,
+                 const double *__restrict__ ref_params, int size, int ring_pass,
+                 const double *__restrict__ rescale_ptr, int num_iter,
+                 double *__restrict__ rescale_out, unsigned long long *__restrict__ stats) {
+    extern __shared__ __align__(16) unsigned char ps_raw[];
+    float4 *r32 = reinterpret_cast<float4 *>(ps_raw);   // populated states, FP32 hi + lo, scaled
+    double *re = reinterpret_cast<double *>(r32 + cap);  // r of every state, then the populated
+    double *im = re + cap;
+    float *k32 = reinterpret_cast<float *>(im + cap);
+    short *idx = reinterpret_cast<short *>(k32 + cap);
+    __shared__ double scratch[5][PS_VIRT * PS_WARPS];
+    __shared__ double taylor64[PS_WARPS][4];
+    __shared__ float taylor32[PS_WARPS][2 * PS_ORDER - 4];
+    __shared__ uint2 red_z[PS_WARPS];
+    __shared__ unsigned red_k[PS_WARPS];
+    __shared__ double red_lo[PS_WARPS], red_lo2[PS_WARPS], red_v[PS_WARPS];
+    __shared__ int red_i[PS_WARPS], wsum[PS_WARPS];
+    __shared__ int n_surv, n_fin[2];
+    __shared__ short surv[NCAND], fin[NCAND];
+    __shared__ float ups[NCAND];
+
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const bool ring = ring_pass != 0;
+    const long long mode = blockIdx.y;
+    const long long ip = blockIdx.x;
+    const int t = pixels[ip];
+    const int *hrow = hist + (long long)hist_row[ip] * n_ref * n_modes + mode * n_ref;
+    nstate += mode * n_ref;
+    fconv += mode * (long long)size * size;
+    PixelConsts pc;
+    pixel_consts_q(t, size, pc);
+
+    // set-up: r of every state with frames or photons once, and the plain
+    // search's sums with its bits
+    double sums[4][PS_VIRT], tot[4];
+#pragma unroll
+    for (int v = 0; v < PS_VIRT; ++v) {
+        sums[0][v] = sums[1][v] = sums[2][v] = sums[3][v] = 0.;
+        for (int s = tid + v * PS_THREADS; s < n_ref; s += PT_THREADS) {
+            const int ns = nstate[s], h = hrow[s];
+            sums[0][v] += (double)ns;
+            sums[1][v] += (double)h;
+            if (ns > 0 || h > 0) {
+                const double2 r = fref_value(pc.qx, pc.qy, pc.qrad, ref_params[3 * s],
+                                             ref_params[3 * s + 1], ref_params[3 * s + 2]);
+                re[s] = r.x;
+                im[s] = r.y;
+                if (ns > 0) {
+                    sums[2][v] = fma((double)ns, r.x, sums[2][v]);
+                    sums[3][v] = fma((double)ns, r.y, sums[3][v]);
+                }
+            }
+        }
+    }
+    virtual_block_sums<4>(sums, tot, scratch);
+    const double dn = tot[0];
+    if (dn == 0.) {  // no frame chose this mode: its model stays as it is
+        if (tid == 0 && rescale_out) rescale_out[mode * n_pix + ip] = NAN;
+        return;
+    }
+    pc.ksum = tot[1];
+    pc.ar = tot[2] / dn;
+    pc.ai = tot[3] / dn;
+    double sq[1][PS_VIRT], var[1];
+#pragma unroll
+    for (int v = 0; v < PS_VIRT; ++v) {
+        sq[0][v] = 0.;
+        for (int s = tid + v * PS_THREADS; s < n_ref; s += PT_THREADS) {
+            const int ns = nstate[s];
+            if (ns > 0) {
+                const double er = xsub(re[s], pc.ar), ei = xsub(im[s], pc.ai);
+                sq[0][v] = fma((double)ns, fma(er, er, xmul(ei, ei)), sq[0][v]);
+            }
+        }
+    }
+    virtual_block_sums<1>(sq, var, scratch + 4);
+    pc.var = var[0] / dn;
+
+    // populated states in order, to the front of re / im (a state's place is
+    // never behind it), with the largest |r| component and count
+    int npop = 0;
+    double rl = 0.;
+    int big = 0;
+    for (int s0 = 0; s0 < n_ref; s0 += PS_THREADS) {
+        const int s = s0 + tid;
+        const int h = s < n_ref ? hrow[s] : 0;
+        double2 r = make_double2(0., 0.);
+        if (h > 0) r = make_double2(re[s], im[s]);
+        const unsigned bal = __ballot_sync(RSPI_FULL_MASK, h > 0);
+        if (lane == 0) wsum[wid] = __popc(bal);
+        __syncthreads();   // counts in place; this round's r are in registers
+        int before = 0, round = 0;
+#pragma unroll
+        for (int w = 0; w < PS_WARPS; ++w) {
+            if (w < wid) before += wsum[w];
+            round += wsum[w];
+        }
+        if (h > 0) {
+            const int pos = npop + before + __popc(bal & ((1u << lane) - 1u));
+            re[pos] = r.x;
+            im[pos] = r.y;
+            k32[pos] = (float)h;
+            idx[pos] = (short)s;
+            rl = fmax(rl, fmax(fabs(r.x), fabs(r.y)));
+            big |= h >= 16777216;
+        }
+        npop += round;
+        __syncthreads();   // wsum's readers are done
+    }
+
+    const double kmean = pc.ksum / dn;
+    const double rescale = ring ? 0. : rescale_ptr[mode];
+    double2 f = fconv[t];
+    double step = hypot(f.x, f.y) / 4.;
+    const double shrink = 33. / 5.;  // sqrt(1089) / 5, maxLP.py:177
+    const bool no_photons = ring && pc.ksum == 0.;
+
+    // FP32 copies of the populated states, scaled by 2^-sexp so that the
+    // largest of |f|_inf and max |r|_inf lies in [1/2, 1)
+    ScreenConsts sk32;
+    bool screen = false;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) rl = fmax(rl, __shfl_xor_sync(RSPI_FULL_MASK, rl, o));
+    if (lane == 0) red_v[wid] = rl;
+    if (tid == 0) n_surv = n_fin[0] = n_fin[1] = 0;
+    big = __syncthreads_or(big);
+#pragma unroll
+    for (int w = 0; w < PS_WARPS; ++w) rl = fmax(rl, red_v[w]);
+    const double top = fmax(rl, fmax(fabs(f.x), fabs(f.y)));
+    if (!no_photons && !big && top > 0x1p-1000 && top < 0x1p1000) {
+        int sexp = 0;
+        frexp(top, &sexp);
+        sk32.ksum = pc.ksum;
+        sk32.inv_dn = 1. / dn;
+        sk32.lr_main = ring ? 0. : log(rescale);
+        sk32.sc = ldexp(1., -sexp);
+        sk32.rinf = rl * sk32.sc;
+        sk32.e2 = 2. * (double)sexp;
+        sk32.ring = ring;
+        for (int j = tid; j < npop; j += PS_THREADS) {
+            const double xr = re[j] * sk32.sc, xi = im[j] * sk32.sc;
+            const float hr = (float)xr, hi = (float)xi;
+            r32[j] = make_float4(hr, hi, (float)(xr - (double)hr), (float)(xi - (double)hi));
+        }
+        screen = true;
+    }
+    __syncthreads();
+
+    const bool taylor_ok = screen && (ring ? kmean > 0. : rescale > 0.) &&
+                           isfinite(ring ? kmean : sk32.lr_main);
+    const int cell = min(tid, PS_CELLS - 1);
+    const int crow = 3 * (cell / 11) + 1, ccol = 3 * (cell % 11) + 1;   // the cell's centre
+    for (int it = 0; it < num_iter; ++it) {
+        double best = -INFINITY;
+        int bidx = 0x7fffffff;
+        // 0. every candidate near f against every z: the expansion
+        const double reach = 8. * step;
+        float zlo = INFINITY, zhi = 0.f;   // bounds of |z|^2 over the states
+        if (taylor_ok) {
+            for (int j = tid; j < npop; j += PS_THREADS) {
+                const double x = f.x + re[j], y = f.y + im[j], g = fma(x, x, y * y);
+                zlo = fminf(zlo, __double2float_rd(g));
+                zhi = fmaxf(zhi, __double2float_ru(g));
+            }
+            // non-negative floats order as their bits
+            const unsigned lo = __reduce_min_sync(RSPI_FULL_MASK, __float_as_uint(zlo));
+            const unsigned hi = __reduce_max_sync(RSPI_FULL_MASK, __float_as_uint(zhi));
+            if (lane == 0) red_z[wid] = make_uint2(lo, hi);
+            __syncthreads();
+#pragma unroll
+            for (int w = 0; w < PS_WARPS; ++w) {
+                zlo = fminf(zlo, __uint_as_float(red_z[w].x));
+                zhi = fmaxf(zhi, __uint_as_float(red_z[w].y));
+            }
+        }
+        // |d| <= sqrt(2) reach <= |z| / 8, in the FP32 range (an empty list:
+        // zlo = inf, zhi = 0)
+        const bool expand = taylor_ok && 128.001 * reach * reach <= (double)zlo &&
+                            zhi < 0x1p100f && zlo > 0x1p-100f && reach > 0x1p-100;
+        // a list of finalists in fin / n_fin[it & 1]; its other counter is
+        // cleared for the next iteration behind this one's first barrier,
+        // which every reader of it has passed
+        const bool listed = step != 0. && screen;
+        bool compare = false;   // threads hold candidates of their own
+        if (screen && step == 0.) {
+            bidx = 0;   // every candidate is f itself: the first index
+            if (stats && tid == 0) atomicAdd(&stats[0], 1ull);
+        } else if (expand) {
+            // sum k (reach / z)^m: m = 1, 2 in FP64 (they meet the quadratic
+            // terms of the mean intensity), the others in FP32
+            double c1[4] = {0., 0., 0., 0.};
+            float cf[2 * PS_ORDER - 4];
+#pragma unroll
+            for (int m = 0; m < 2 * PS_ORDER - 4; ++m) cf[m] = 0.f;
+            for (int j = tid; j < npop; j += PS_THREADS) {
+                const double x = f.x + re[j], y = f.y + im[j];
+                const double ig = reach / fma(x, x, y * y), kj = (double)k32[j];
+                const double wr = x * ig, wi = -y * ig;   // reach / z
+                const double vr = fma(wr, wr, -wi * wi), vi = 2. * wr * wi;
+                c1[0] = fma(kj, wr, c1[0]);
+                c1[1] = fma(kj, wi, c1[1]);
+                c1[2] = fma(kj, vr, c1[2]);
+                c1[3] = fma(kj, vi, c1[3]);
+                const float fr = (float)wr, fi = (float)wi;
+                float pr = (float)(kj * vr), pi = (float)(kj * vi);
+#pragma unroll
+                for (int m = 0; m < PS_ORDER - 2; ++m) {
+                    const float tr = pr * fr - pi * fi;
+                    pi = pr * fi + pi * fr;
+                    pr = tr;
+                    cf[2 * m] += pr;
+                    cf[2 * m + 1] += pi;
+                }
+            }
+            if (wid * 32 < npop) {
+#pragma unroll
+                for (int m = 0; m < 4; ++m) c1[m] = warp_sum(c1[m]);
+#pragma unroll
+                for (int m = 0; m < 2 * PS_ORDER - 4; ++m) cf[m] = warp_sum(cf[m]);
+            }
+            if (lane == 0) {
+#pragma unroll
+                for (int m = 0; m < 4; ++m) taylor64[wid][m] = c1[m];
+#pragma unroll
+                for (int m = 0; m < 2 * PS_ORDER - 4; ++m) taylor32[wid][m] = cf[m];
+            }
+            __syncthreads();
+            if (tid == 0) n_fin[(it + 1) & 1] = 0;
+            // value relative to f's, at d = reach (dx, dy):
+            //   lx dx + ly dy + Re(d^2 (c_2 + c_3 d + ...)) - vq |d|^2
+            // (ring: - K/n (log1p(t) - t), t = mw(d) / mw - 1),
+            //   c_m = 2 (-1)^(m+1) / m sum k (reach / z)^m / n
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+                c1[m] = taylor64[0][m];
+#pragma unroll
+                for (int w = 1; w < PS_WARPS; ++w) c1[m] += taylor64[w][m];
+            }
+            const float invn = (float)sk32.inv_dn;
+#pragma unroll
+            for (int m = 0; m < PS_ORDER - 2; ++m) {
+                const float c = (m & 1 ? -2.f : 2.f) / (float)(m + 3) * invn;
+                float tr = taylor32[0][2 * m], ti = taylor32[0][2 * m + 1];
+#pragma unroll
+                for (int w = 1; w < PS_WARPS; ++w) {
+                    tr += taylor32[w][2 * m];
+                    ti += taylor32[w][2 * m + 1];
+                }
+                cf[2 * m] = c * tr;
+                cf[2 * m + 1] = c * ti;
+            }
+            const double er = f.x + pc.ar, ei = f.y + pc.ai;
+            const double mw0 = fma(er, er, fma(ei, ei, pc.var)), kn64 = sk32.ksum * sk32.inv_dn;
+            const double mt = 1. / mw0, mf = ring ? kn64 * mt : rescale;
+            const float lx = (float)(2. * c1[0] * sk32.inv_dn - 2. * mf * reach * er);
+            const float ly = (float)(-2. * c1[1] * sk32.inv_dn - 2. * mf * reach * ei);
+            const float c2r = (float)(-c1[2] * sk32.inv_dn), c2i = (float)(-c1[3] * sk32.inv_dn);
+            const float vq = (float)(mf * reach * reach), kn = (float)kn64;
+            const float tx = (float)(2. * mt * reach * er), ty = (float)(2. * mt * reach * ei);
+            const float tq = (float)(mt * reach * reach), tabs = fabsf(tx) + fabsf(ty) + 2.f * tq;
+            const float rz = npop > 0 ? (float)(reach * reach / (double)zlo) : 0.f;
+            // errors: the FP64 rounding of the plain search's values (2^-40
+            // of their terms, |ln |z|^2| from the exponents), the FP32
+            // arithmetic here (2^-19 of the first two orders' terms, 2^-17
+            // of the others', below 2.3 K/n (reach / |z|)^3), and beyond
+            // order 8 the sum of 2 k |d / z|^m / m, below 0.032 K/n (|d| / |z|)^8
+            const float lz =
+                npop > 0 ? 0.7f * (float)(max(abs(ilogbf(zlo)), abs(ilogbf(zhi))) + 2) : 0.f;
+            const float lr = (float)(ring ? fabs(log(kmean * mt)) : fabs(sk32.lr_main));
+            const float base =
+                0x1p-40f * (kn * (lr + lz + 2.f) + (float)(mf * mw0) * (2.f + 2.f * tabs)) +
+                0x1p-19f * (fabsf(lx) + fabsf(ly) + 2.f * (fabsf(c2r) + fabsf(c2i) + vq)) +
+                0x1p-17f * 2.3f * kn * rz * sqrtf(rz);
+            float tl = -INFINITY;
+            for (int c = tid; c < NCAND; c += PS_THREADS) {
+                const int row = c / 33;
+                const float dx = -1.f + 0.0625f * (float)row;
+                const float dy = -1.f + 0.0625f * (float)(c - 33 * row);
+                float ar = cf[2 * PS_ORDER - 6], ai = cf[2 * PS_ORDER - 5];
+#pragma unroll
+                for (int m = PS_ORDER - 4; m >= 0; --m) {
+                    const float tr = fmaf(ar, dx, fmaf(-ai, dy, cf[2 * m]));
+                    ai = fmaf(ar, dy, fmaf(ai, dx, cf[2 * m + 1]));
+                    ar = tr;
+                }
+                const float tr = fmaf(ar, dx, fmaf(-ai, dy, c2r));
+                ai = fmaf(ar, dy, fmaf(ai, dx, c2i));
+                const float dd = fmaf(dx, dx, dy * dy);
+                float v = fmaf(lx, dx, ly * dy) +
+                          (tr * fmaf(dx, dx, -dy * dy) - 2.f * ai * dx * dy - vq * dd);
+                float r2 = rz * dd;
+                r2 *= r2;
+                float e = fmaf(kn * 0.032f, r2 * r2, base);
+                if (ring) {
+                    const float tt = fmaf(tx, dx, fmaf(ty, dy, tq * dd));
+                    v -= kn * (log1pf(tt) - tt);
+                    e += 0x1p-20f * kn * tabs * (1.f + rcp_approx(1.f + tt));
+                }
+                tl = fmaxf(tl, v - e);   // a NaN (no bound) does not count
+                ups[c] = v + e;
+            }
+            unsigned key = __float_as_uint(tl);
+            key = (key & 0x80000000u) ? ~key : key | 0x80000000u;
+            key = __reduce_max_sync(RSPI_FULL_MASK, key);
+            if (lane == 0) red_k[wid] = key;
+            __syncthreads();
+#pragma unroll
+            for (int w = 0; w < PS_WARPS; ++w) key = max(key, red_k[w]);
+            tl = __uint_as_float((key & 0x80000000u) ? key & 0x7fffffffu : ~key);
+            for (int c0 = 0; c0 < NCAND; c0 += PS_THREADS) {
+                const int c = c0 + tid;
+                list_add(c < NCAND && !(ups[c] < tl), (short)c, fin, &n_fin[it & 1]);
+            }
+            __syncthreads();
+        } else if (screen) {
+            // 1. cell centres
+            const Cand cd = cand_at(crow * 33 + ccol, f, step, pc, ring, kmean, rescale);
+            float gmin = INFINITY, hsum = 0.f;
+            float2 gsum = make_float2(0.f, 0.f);
+            double a = 0., b = 0.;
+            {
+                const double xs = cd.fr * sk32.sc, ys = cd.fi * sk32.sc;
+                const float2 xh = make_float2((float)xs, (float)ys);
+                const float2 xl = make_float2((float)(xs - (double)xh.x), (float)(ys - (double)xh.y));
+                for (int j0 = 0; j0 < npop; j0 += PT_CHUNK) {
+                    float2 ab = make_float2(0.f, 0.f);
+                    const int j1 = min(npop, j0 + PT_CHUNK);
+#pragma unroll 4
+                    for (int j = j0; j < j1; ++j) {
+                        const float kj = k32[j];
+                        float2 z;
+                        const float g = screen_term(xh, xl, r32[j], kj, gmin, ab, z);
+                        const float w = kj * rcp_approx(g);
+                        hsum += w;
+                        gsum = __ffma2_rn(make_float2(w, w), z, gsum);
+                    }
+                    a += (double)ab.x;
+                    b += (double)ab.y;
+                }
+            }
+            double q = 0., e = 0., fm = 0., amax = 0.;
+            const bool ok = cand_bound(cd, a, b, gmin, sk32, q, e, fm, amax);
+            double tl = ok ? q - e : -INFINITY;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) tl = fmax(tl, __shfl_xor_sync(RSPI_FULL_MASK, tl, o));
+            if (lane == 0) red_lo[wid] = tl;
+            __syncthreads();
+#pragma unroll
+            for (int w = 0; w < PS_WARPS; ++w) tl = fmax(tl, red_lo[w]);
+            if (tid == 0) n_fin[(it + 1) & 1] = 0;
+            unsigned keep = 0;   // the cell's nine candidates, bit 3 (row + 1) + (col + 1)
+            if (tid < PS_CELLS) {
+                const double h = 0.5 * step, hsd = h * sk32.sc;
+                if (!ok || !(hsd >= 0x1p-30 * amax)) {
+                    keep = 0x1ffu;
+                } else {
+                    const float invn = (float)sk32.inv_dn, hs = (float)hsd;
+                    const float ux = 2.f * hs * gsum.x * invn, uy = 2.f * hs * gsum.y * invn;
+                    const float uq = hs * hs * hsum * invn;
+                    const double er = cd.fr + pc.ar, ei = cd.fi + pc.ai;
+                    // of the mean-intensity term: rho (2 d.e + |d|^2); of the
+                    // ring's rescale: mw(d) / mw - 1 = (2 d.e + |d|^2) / mw
+                    const double m = ring ? 1. / cd.mw : cd.rho;
+                    const float vx = (float)(2. * m * h * er), vy = (float)(2. * m * h * ei);
+                    const float vq = (float)(m * h * h);
+                    const float kn = (float)(sk32.ksum * sk32.inv_dn);
+                    const float vabs = fabsf(vx) + fabsf(vy) + 2.f * vq;
+                    float slack = (float)(1.000001 * e + 0x1p-30 * (fm + 2. * cd.rho * h * h));
+                    slack += 0x1p-13f * (3.f * hs * invn * sqrtf((float)sk32.ksum * hsum) + 2.f * uq);
+                    if (!ring) slack += 0x1p-18f * vabs;
+                    const double gap = tl - q;
+                    const float lim = (float)(gap - 0x1p-22 * fabs(gap));
+#pragma unroll
+                    for (int k = 0; k < 9; ++k) {
+                        const float dx = (float)(k / 3 - 1), dy = (float)(k % 3 - 1);
+                        const float dd = dx * dx + dy * dy;
+                        float u = dx * ux + dy * uy + dd * uq;
+                        if (!ring) {
+                            u -= dx * vx + dy * vy + dd * vq;
+                        } else {
+                            // -K/n ln(mw(d) / mw), its argument taken low
+                            const float w = 1.f + (dx * vx + dy * vy + dd * vq) -
+                                            0x1p-18f * (1.f + vabs);
+                            const float l = lg2_approx(w);   // NaN where w < 0: kept
+                            u -= kn * 0.69314718f * (l - 0x1p-20f - 0x1p-20f * fabsf(l));
+                        }
+                        if (!(u + slack < lim)) keep |= 1u << k;
+                    }
+                }
+            }
+            {
+                int pos = list_push(__popc(keep), &n_surv);
+                for (unsigned m = keep; m; m &= m - 1) {
+                    const int k = __ffs(m) - 1;
+                    surv[pos++] = (short)((crow + k / 3 - 1) * 33 + ccol + k % 3 - 1);
+                }
+            }
+            __syncthreads();
+            // 2. the survivors, four threads each (a thread each beyond a pass)
+            const int ns = n_surv;
+            const int split = ns <= PS_THREADS / 4 ? 4 : 1, part = tid & (split - 1);
+            for (int i0 = 0; i0 < ns; i0 += PS_THREADS / split) {
+                const int i = i0 + tid / split;
+                const Cand cs = cand_at(surv[min(i, ns - 1)], f, step, pc, ring, kmean, rescale);
+                const double xs = cs.fr * sk32.sc, ys = cs.fi * sk32.sc;
+                const float2 xh = make_float2((float)xs, (float)ys);
+                const float2 xl = make_float2((float)(xs - (double)xh.x), (float)(ys - (double)xh.y));
+                float gm = INFINITY;
+                double as = 0., bs = 0.;
+                for (int j0 = part; j0 < npop; j0 += split * PT_CHUNK) {
+                    float2 ab = make_float2(0.f, 0.f);
+                    const int j1 = min(npop, j0 + split * PT_CHUNK);
+#pragma unroll 2
+                    for (int j = j0; j < j1; j += split) {
+                        float2 z;
+                        screen_term(xh, xl, r32[j], k32[j], gm, ab, z);
+                    }
+                    as += (double)ab.x;
+                    bs += (double)ab.y;
+                }
+                if (split == 4) {
+#pragma unroll
+                    for (int o = 1; o < 4; o <<= 1) {
+                        as += __shfl_xor_sync(RSPI_FULL_MASK, as, o);
+                        bs += __shfl_xor_sync(RSPI_FULL_MASK, bs, o);
+                        gm = fminf(gm, __shfl_xor_sync(RSPI_FULL_MASK, gm, o));
+                    }
+                }
+                double qs, es, fs, am;
+                const bool oks = cand_bound(cs, as, bs, gm, sk32, qs, es, fs, am);
+                if (oks) tl = fmax(tl, qs - es);
+                if (part == 0 && i < ns) ups[i] = oks ? __double2float_ru(qs + es) : INFINITY;
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) tl = fmax(tl, __shfl_xor_sync(RSPI_FULL_MASK, tl, o));
+            if (lane == 0) red_lo2[wid] = tl;
+            __syncthreads();
+#pragma unroll
+            for (int w = 0; w < PS_WARPS; ++w) tl = fmax(tl, red_lo2[w]);
+            for (int i0 = 0; i0 < ns; i0 += PS_THREADS) {
+                const int i = i0 + tid;
+                const bool hit = i < ns && (double)ups[i] >= tl;
+                list_add(hit, hit ? surv[i] : (short)0, fin, &n_fin[it & 1]);
+            }
+            __syncthreads();
+            if (tid == 0) n_surv = 0;
+        } else {
+            if (no_photons) {
+                bidx = 0;   // 0 * log(0) in every frame: NaN, the first index
+            } else {
+                plain_candidates(nullptr, NCAND, f, step, pc, ring, kmean, rescale, dn, npop, re,
+                                 im, idx, hrow, best, bidx);
+                compare = true;
+            }
+            if (stats && tid == 0) atomicAdd(&stats[1], 1ull);
+        }
+        // 3. the finalists in FP64: thread p of four sums the states j = p
+        // mod 4 in order, as the plain search's partial sums
+        const int nf = listed ? n_fin[it & 1] : 0;
+        if (nf == 1) {
+            bidx = fin[0];   // nothing to compare it with
+        } else if (nf > 1) {
+            compare = true;
+            if (nf <= PS_THREADS / NPART) {
+                const int part = tid % NPART, i = tid / NPART;
+                const int c = fin[min(i, nf - 1)];
+                const Cand cc = cand_at(c, f, step, pc, ring, kmean, rescale);
+                double acc = 0.;
+                if (i < nf)
+                    for (int j = part; j < npop; j += NPART)
+                        acc = term64(acc, (double)k32[j], cc, re[j], im[j]);
+                const double v1 = __shfl_down_sync(RSPI_FULL_MASK, acc, 1);
+                const double v2 = __shfl_down_sync(RSPI_FULL_MASK, acc, 2);
+                const double v3 = __shfl_down_sync(RSPI_FULL_MASK, acc, 3);
+                if (i < nf && part == 0) {
+                    best = cand_q(combine4(acc, v1, v2, v3), dn, cc);
+                    bidx = c;
+                }
+            } else {
+                plain_candidates(fin, nf, f, step, pc, ring, kmean, rescale, dn, npop, re, im,
+                                 idx, hrow, best, bidx);
+            }
+        }
+        if (nf > 0 && stats && tid == 0) {
+            atomicAdd(&stats[0], 1ull);
+            atomicAdd(&stats[2], (unsigned long long)nf);
+        }
+        if (compare) {   // the CTA's argmax
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const double ov = __shfl_xor_sync(RSPI_FULL_MASK, best, o);
+                const int oi = __shfl_xor_sync(RSPI_FULL_MASK, bidx, o);
+                if (argmax_better(ov, oi, best, bidx)) {
+                    best = ov;
+                    bidx = oi;
+                }
+            }
+            __syncthreads();   // the previous iteration's readers of red_v, red_i
+            if (lane == 0) {
+                red_v[wid] = best;
+                red_i[wid] = bidx;
+            }
+            __syncthreads();
+            best = red_v[0];
+            bidx = red_i[0];
+#pragma unroll
+            for (int w = 1; w < PS_WARPS; ++w)
+                if (argmax_better(red_v[w], red_i[w], best, bidx)) {
+                    best = red_v[w];
+                    bidx = red_i[w];
+                }
+        }
+        const double px = -8. + 0.5 * (bidx / 33), py = -8. + 0.5 * (bidx % 33);
+        const double2 fnew = make_double2(xadd(f.x, xmul(px, step)), xadd(f.y, xmul(py, step)));
+        const double step_new = bidx == CENTRE ? step / shrink : step;
+        // step_new / |fnew| < 1e-3 keeps f (maxLP.py:162-165); the quotient
+        // itself only where the squares leave it open
+        const double h2 = fma(fnew.x, fnew.x, fnew.y * fnew.y), s2 = step_new * step_new;
+        const bool far = h2 > 0x1p-900 && h2 < 0x1p900 && s2 > 0x1p-900;
+        if (far && s2 < 0.999999e-6 * h2) break;
+        if (!(far && s2 > 1.000001e-6 * h2) && step_new / hypot(fnew.x, fnew.y) < 1.e-3) break;
+        f = fnew;
+        step = step_new;
+    }
+    if (tid == 0) {
         fconv[t] = f;
         if (rescale_out) {   // maxLP.py:328, with the candidates' explicit roundings
             const double er = xadd(f.x, pc.ar), ei = xadd(f.y, pc.ai);
@@ -1136,7 +1617,7 @@ extern "C" int rspi_maxlp_pattern(double *fconv, const int *pixels, const int *h
         (rescale_mode == 1 && !rescale) || (rescale_mode != 0 && rescale_mode != 1))
         return RSPI_ERR_ARG;
     const dim3 grid((unsigned)n_pix, (unsigned)n_modes);
-    k_pattern<false><<<grid, PT_THREADS, 0, stream>>>(
+    k_pattern<<<grid, PT_THREADS, 0, stream>>>(
         (double2 *)fconv, pixels, hist_row, n_pix, hist, n_ref, nstate, n_modes, ref_params,
         (int)size, rescale_mode == 0, rescale, num_iter, rescale_out, nullptr);
     RSPI_RETURN_LAUNCH();
@@ -1156,9 +1637,19 @@ extern "C" int rspi_maxlp_pattern_screened(double *fconv, const int *pixels, con
         (rescale_mode == 1 && !rescale) || (rescale_mode != 0 && rescale_mode != 1))
         return RSPI_ERR_ARG;
     const dim3 grid((unsigned)n_pix, (unsigned)n_modes);
-    k_pattern<true><<<grid, PT_THREADS, 0, stream>>>(
-        (double2 *)fconv, pixels, hist_row, n_pix, hist, n_ref, nstate, n_modes, ref_params,
-        (int)size, rescale_mode == 0, rescale, num_iter, rescale_out, stats);
+    if (n_ref > POP_CAP) {   // the populated states may not fit: the plain search
+        k_pattern<<<grid, PT_THREADS, 0, stream>>>(
+            (double2 *)fconv, pixels, hist_row, n_pix, hist, n_ref, nstate, n_modes, ref_params,
+            (int)size, rescale_mode == 0, rescale, num_iter, rescale_out, stats);
+        RSPI_RETURN_LAUNCH();
+    }
+    const int cap = ((int)n_ref + 7) / 8 * 8;
+    const size_t smem = (size_t)cap * ps_state_bytes();
+    static RspiSmemOptIn optin;
+    if (!rspi_smem_optin((const void *)k_pattern_screen, smem, optin)) return RSPI_ERR_CUDA;
+    k_pattern_screen<<<grid, PS_THREADS, smem, stream>>>(
+        (double2 *)fconv, pixels, hist_row, n_pix, hist, (int)n_ref, cap, nstate, n_modes,
+        ref_params, (int)size, rescale_mode == 0, rescale, num_iter, rescale_out, stats);
     RSPI_RETURN_LAUNCH();
 }
 
