@@ -712,6 +712,30 @@ int rspi_nll(int precision, int want_grad, const int *ones, const int *multi,
              const double *scale, double *nll, double *gfre, double *gfim, double *gdia,
              double *gsx, double *gsy, double *gscale, int *err, cudaStream_t stream);
 
+/* rspi_nll for the pixels of a whole ring on the detector's grid, q = (x - c,
+ * y - c) / size with c = size / 2, with the dense part's reference amplitudes
+ * from tables.  The n_pix pixels (rows m of fre .. qrad) are n_pix / 4 orbits
+ * of the quarter turn about c: orbit i holds rows order[4 i .. 4 i + 3] for
+ * (x, y), (-y, x), (-x, -y), (y, -x) relative to c, with x >= 1 and y >= 0 in
+ * xy[i] = x << 16 | y.  Orbits are grouped rspi_nll_grid_tile(precision,
+ * size) at a time; rad_id[i] numbers the orbit's radius among the distinct
+ * ones, rad_q[] holds those (the pixels' qrad), and tile_rads bounds the span
+ * (last - first + 1) of a group's rad_id.  order on a 16-byte boundary.
+ * Sizes whose tables exceed shared memory: RSPI_ERR_ARG. */
+int rspi_nll_grid(int precision, int want_grad, const int *ones, const int *multi,
+             const long long *ones_accum, const long long *multi_accum, const int *place_ones,
+             const int *place_multi, const int *count_multi, long long n_frames,
+             const double *rot_cs, long long size, const int *mask_idx, long long n_pix, const int *order,
+                  const int *xy, const int *rad_id, const double *rad_q, int tile_rads,
+             const double *fre, const double *fim, const double *qx, const double *qy,
+             const double *qrad, const double *dia, const double *sx, const double *sy,
+             const double *scale, double *nll, double *gfre, double *gfim, double *gdia,
+             double *gsx, double *gsy, double *gscale, int *err, cudaStream_t stream);
+
+/* Orbits per group of rspi_nll_grid for a size^2 detector; -1: a detector too
+ * large for its tables (rspi_nll takes it), or an unknown precision. */
+int rspi_nll_grid_tile(int precision, long long size);
+
 /* The E-step side of the adjoint: negative log-likelihood through model
  * slicing for frames in given orientations (rot_cs[2d], rot_cs[2d + 1]: the
  * cos, sin of frame d's angle, as rspi_rot_log_slices uses them) with
@@ -729,6 +753,20 @@ int rspi_nll(int precision, int want_grad, const int *ones, const int *multi,
  * reference, which has no gradient of its likelihood. */
 int rspi_emc_nll(int precision, int want_grad, const double *model, long long size,
                  const double *bg, const int *sel_pix, long long n_sel, const int *pix2sel,
+                 const int *ones, const int *multi, const long long *ones_accum,
+                 const long long *multi_accum, const int *place_ones, const int *place_multi,
+                 const int *count_multi, long long n_frames, const double *rot_cs,
+                 const double *dia, const double *sx, const double *sy, const double *scale,
+                 double vscale, double *nll, double *gre, double *gim, double *gdia,
+                 double *gsx, double *gsy, double *gscale, int *err, cudaStream_t stream);
+
+/* rspi_emc_nll with the masked sum's reference amplitudes from rspi_nll_grid's
+ * tables of the likelihood pixels (order holds flat pixel numbers, rad_q the
+ * radii over size), and bg_sum their background's sum. */
+int rspi_emc_nll_grid(int precision, int want_grad, const double *model, long long size,
+                 const double *bg, const int *sel_pix, long long n_sel, const int *order,
+                      const int *xy, const int *rad_id, const double *rad_q, int tile_rads,
+                      double bg_sum, const int *pix2sel,
                  const int *ones, const int *multi, const long long *ones_accum,
                  const long long *multi_accum, const int *place_ones, const int *place_multi,
                  const int *count_multi, long long n_frames, const double *rot_cs,

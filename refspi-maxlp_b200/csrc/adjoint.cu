@@ -19,6 +19,7 @@
 // CT is the arithmetic type of the terms (float: the production FP32 form;
 // double: the FP64 form used by the finite-difference checks); every sum is
 // accumulated in FP64.
+#include "nll_grid.cuh"
 #include "rspi_common.cuh"
 
 namespace {
@@ -140,7 +141,7 @@ k_nll_dense(const double *__restrict__ fre, const double *__restrict__ fim,
 
 // Photon part: one warp per frame, lanes over its photons; each photon goes
 // to every phaser pixel whose exact rotated index lands on it.
-template <typename CT, bool GRAD>
+template <typename CT, bool GRAD, bool GRID>
 __global__ void __launch_bounds__(256)
 k_nll_photons(const int *__restrict__ ones, const int *__restrict__ multi,
               const long long *__restrict__ ones_accum, const long long *__restrict__ multi_accum,
@@ -182,33 +183,34 @@ k_nll_photons(const int *__restrict__ ones, const int *__restrict__ multi,
             }
             const int ux = p / size, uy = p - (p / size) * size;
             // model pixels near the inverse image (3x3), checked with the forward map
-            const double vx = (double)ux - c0, vy = (double)uy - c0;
-            const int bx = (int)rint(c * vx + s * vy + c0);
-            const int by = (int)rint(-s * vx + c * vy + c0);
-            for (int ax = -1; ax <= 1; ++ax)
-                for (int ay = -1; ay <= 1; ++ay) {
-                    const int tx = bx + ax, ty = by + ay;
-                    if (tx < 0 || ty < 0 || tx >= size || ty >= size) continue;
-                    const int m = mask_idx[tx * size + ty];
-                    if (m < 0) continue;
-                    int ox, oy;
+            int bx, by;
+            for (unsigned near = near_pixels(ux, uy, c, s, c0, bx, by); near; near &= near - 1) {
+                const int nk = __ffs(near) - 1;
+                const int tx = bx + nk / 3 - 1, ty = by + nk % 3 - 1;
+                if (tx < 0 || ty < 0 || tx >= size || ty >= size) continue;
+                const int m = mask_idx[tx * size + ty];
+                if (m < 0) continue;
+                int ox, oy;
+                if (GRID)   // qx, qy are the grid's quotients
+                    forward_q(qx[m], qy[m], c, s, size, ox, oy);
+                else
                     forward_pixel(tx, ty, c, s, size, ox, oy);
-                    if (ox != ux || oy != uy) continue;
-                    const Ref<CT> r = ref_amp<CT>((CT)qx[m], (CT)qy[m], (CT)qrad[m], dd, xd, yd);
-                    const CT zr = (CT)fre[m] + r.rr, zi = (CT)fim[m] + r.ri;
-                    const CT a = zr * zr + zi * zi;
-                    const CT k = (CT)cnt;
-                    nll -= (double)k * log((double)(sd * a));
-                    if (GRAD) {
-                        const CT wr = (CT)2 * k * zr / a, wi = (CT)2 * k * zi / a;
-                        atomicAdd(&gfre[m], -(double)wr);
-                        atomicAdd(&gfim[m], -(double)wi);
-                        ga -= (double)(k / sd);
-                        gd -= (double)(wr * r.dd_r + wi * r.dd_i);
-                        gx -= (double)(wr * r.dx_r + wi * r.dx_i);
-                        gy -= (double)(wr * r.dy_r + wi * r.dy_i);
-                    }
+                if (ox != ux || oy != uy) continue;
+                const Ref<CT> r = ref_amp<CT>((CT)qx[m], (CT)qy[m], (CT)qrad[m], dd, xd, yd);
+                const CT zr = (CT)fre[m] + r.rr, zi = (CT)fim[m] + r.ri;
+                const CT a = zr * zr + zi * zi;
+                const CT k = (CT)cnt;
+                nll -= (double)k * log((double)(sd * a));
+                if (GRAD) {
+                    const CT wr = (CT)2 * k * zr / a, wi = (CT)2 * k * zi / a;
+                    atomicAdd(&gfre[m], -(double)wr);
+                    atomicAdd(&gfim[m], -(double)wi);
+                    ga -= (double)(k / sd);
+                    gd -= (double)(wr * r.dd_r + wi * r.dd_i);
+                    gx -= (double)(wr * r.dx_r + wi * r.dx_i);
+                    gy -= (double)(wr * r.dy_r + wi * r.dy_i);
                 }
+            }
         }
         if (GRAD) {
             ga = warp_sum(ga);
@@ -228,26 +230,46 @@ k_nll_photons(const int *__restrict__ ones, const int *__restrict__ multi,
 }
 
 template <typename CT, bool GRAD>
-void launch_all(const int *ones, const int *multi, const long long *oacc, const long long *macc,
+int launch_dense(const GridTables &g, long long n_pix, int size, const double *fre,
+                 const double *fim, const double *qx, const double *qy, const double *qrad,
+                 const double *dia, const double *sx, const double *sy, const double *scale,
+                 long long n_frames, double *out, double *gfre, double *gfim, double *gdia,
+                 double *gsx, double *gsy, double *gscale, cudaStream_t stream) {
+    if (n_pix == 0) return RSPI_OK;
+    if (!g.order) {
+        const dim3 grid((unsigned)((n_pix + 255) / 256),
+                        (unsigned)((n_frames + DT_FRAMES - 1) / DT_FRAMES));
+        k_nll_dense<CT, GRAD><<<grid, 256, 0, stream>>>(fre, fim, qx, qy, qrad, n_pix, dia, sx,
+                                                         sy, scale, n_frames, out, gfre, gfim,
+                                                         gdia, gsx, gsy, gscale);
+        return RSPI_OK;
+    }
+    return launch_dense_grid<CT, GRAD>(g, n_pix, size, fre, fim, 1, 1., 0., dia, sx, sy, scale,
+                                       n_frames, out, gfre, gfim, gdia, gsx, gsy, gscale, stream);
+}
+
+template <typename CT, bool GRAD>
+int launch_all(const GridTables &g, const int *ones, const int *multi, const long long *oacc, const long long *macc,
                 const int *po, const int *pm, const int *cm, long long n_frames,
                 const double *rot_cs, int size, const int *mask_idx, long long n_pix,
                 const double *fre, const double *fim, const double *qx, const double *qy,
                 const double *qrad, const double *dia, const double *sx, const double *sy,
                 const double *scale, double *out, double *gfre, double *gfim, double *gdia,
                 double *gsx, double *gsy, double *gscale, int *err, cudaStream_t stream) {
-    const dim3 grid((unsigned)((n_pix + 255) / 256), (unsigned)((n_frames + DT_FRAMES - 1) / DT_FRAMES));
-    if (n_pix > 0)
-        k_nll_dense<CT, GRAD><<<grid, 256, 0, stream>>>(fre, fim, qx, qy, qrad, n_pix, dia, sx,
-                                                         sy, scale, n_frames, out, gfre, gfim,
-                                                         gdia, gsx, gsy, gscale);
-    k_nll_photons<CT, GRAD><<<rspi_blocks(n_frames * 32, 256), 256, 0, stream>>>(
+    const int st = launch_dense<CT, GRAD>(g, n_pix, size, fre, fim, qx, qy, qrad, dia, sx, sy,
+                                          scale, n_frames, out, gfre, gfim, gdia, gsx, gsy,
+                                          gscale, stream);
+    if (st != RSPI_OK) return st;
+    const auto photons = g.order ? k_nll_photons<CT, GRAD, true> : k_nll_photons<CT, GRAD, false>;
+    photons<<<rspi_blocks(n_frames * 32, 256), 256, 0, stream>>>(
         ones, multi, oacc, macc, po, pm, cm, n_frames, rot_cs, size, mask_idx, fre, fim, qx, qy,
         qrad, dia, sx, sy, scale, out, gfre, gfim, gdia, gsx, gsy, gscale, err);
+    RSPI_RETURN_LAUNCH();
 }
 
 }  // namespace
 
-extern "C" int rspi_nll(int precision, int want_grad, const int *ones, const int *multi,
+static int nll_entry(const GridTables &g, int precision, int want_grad, const int *ones, const int *multi,
                         const long long *ones_accum, const long long *multi_accum,
                         const int *place_ones, const int *place_multi, const int *count_multi,
                         long long n_frames, const double *rot_cs, long long size,
@@ -273,13 +295,54 @@ extern "C" int rspi_nll(int precision, int want_grad, const int *ones, const int
         cudaMemsetAsync(gscale, 0, sizeof(double) * n_frames, stream);
     }
 #define RSPI_NLL(CT, G)                                                                          \
-    launch_all<CT, G>(ones, multi, ones_accum, multi_accum, place_ones, place_multi, count_multi, \
+    launch_all<CT, G>(g, ones, multi, ones_accum, multi_accum, place_ones, place_multi, count_multi, \
                       n_frames, rot_cs, (int)size, mask_idx, n_pix, fre, fim, qx, qy, qrad, dia,  \
                       sx, sy, scale, nll, gfre, gfim, gdia, gsx, gsy, gscale, err, stream)
-    if (precision == 1 && want_grad) RSPI_NLL(double, true);
-    else if (precision == 1) RSPI_NLL(double, false);
-    else if (want_grad) RSPI_NLL(float, true);
-    else RSPI_NLL(float, false);
+    if (precision == 1 && want_grad) return RSPI_NLL(double, true);
+    if (precision == 1) return RSPI_NLL(double, false);
+    if (want_grad) return RSPI_NLL(float, true);
+    return RSPI_NLL(float, false);
 #undef RSPI_NLL
-    RSPI_RETURN_LAUNCH();
+}
+
+extern "C" int rspi_nll(int precision, int want_grad, const int *ones, const int *multi,
+                        const long long *ones_accum, const long long *multi_accum,
+                        const int *place_ones, const int *place_multi, const int *count_multi,
+                        long long n_frames, const double *rot_cs, long long size,
+                        const int *mask_idx, long long n_pix, const double *fre,
+                        const double *fim, const double *qx, const double *qy,
+                        const double *qrad, const double *dia, const double *sx,
+                        const double *sy, const double *scale, double *nll, double *gfre,
+                        double *gfim, double *gdia, double *gsx, double *gsy, double *gscale,
+                        int *err, cudaStream_t stream) {
+    const GridTables none{nullptr, nullptr, nullptr, nullptr, 0};
+    return nll_entry(none, precision, want_grad, ones, multi, ones_accum, multi_accum,
+                     place_ones, place_multi, count_multi, n_frames, rot_cs, size, mask_idx,
+                     n_pix, fre, fim, qx, qy, qrad, dia, sx, sy, scale, nll, gfre, gfim, gdia,
+                     gsx, gsy, gscale, err, stream);
+}
+
+extern "C" int rspi_nll_grid_tile(int precision, long long size) {
+    return dense_grid_tile(precision, size);
+}
+
+extern "C" int rspi_nll_grid(int precision, int want_grad, const int *ones, const int *multi,
+                             const long long *ones_accum, const long long *multi_accum,
+                             const int *place_ones, const int *place_multi,
+                             const int *count_multi, long long n_frames, const double *rot_cs,
+                             long long size, const int *mask_idx, long long n_pix,
+                             const int *order, const int *xy, const int *rad_id,
+                             const double *rad_q, int tile_rads, const double *fre,
+                             const double *fim, const double *qx, const double *qy,
+                             const double *qrad, const double *dia, const double *sx,
+                             const double *sy, const double *scale, double *nll, double *gfre,
+                             double *gfim, double *gdia, double *gsx, double *gsy,
+                             double *gscale, int *err, cudaStream_t stream) {
+    if (!grid_tables_ok(precision, size, n_pix, order, xy, rad_id, rad_q, tile_rads))
+        return RSPI_ERR_ARG;
+    const GridTables g{order, xy, rad_id, rad_q, tile_rads};
+    return nll_entry(g, precision, want_grad, ones, multi, ones_accum, multi_accum, place_ones,
+                     place_multi, count_multi, n_frames, rot_cs, size, mask_idx, n_pix, fre, fim,
+                     qx, qy, qrad, dia, sx, sy, scale, nll, gfre, gfim, gdia, gsx, gsy, gscale,
+                     err, stream);
 }

@@ -25,6 +25,7 @@
 // recomputed where needed: nothing frames x pixels is stored.  CT is the
 // arithmetic type of the terms (float: production; double: the form the
 // finite-difference checks use); every sum is FP64.
+#include "nll_grid.cuh"
 #include "rspi_common.cuh"
 
 namespace {
@@ -270,14 +271,20 @@ k_emc_nll_photons(const int *__restrict__ ones, const int *__restrict__ multi,
 }
 
 template <typename CT, bool GRAD>
-void emc_launch(const double2 *model, int size, const double *bg, const int *sel_pix,
+int emc_launch(const GridTables &g, double bg_sum, const double2 *model, int size, const double *bg, const int *sel_pix,
                 long long n_sel, const int *pix2sel, const int *ones, const int *multi,
                 const long long *oacc, const long long *macc, const int *po, const int *pm,
                 const int *cm, long long n_frames, const double *rot_cs, const double *dia,
                 const double *sx, const double *sy, const double *scale, double vscale,
                 double *out, double *gre, double *gim, double *gdia, double *gsx, double *gsy,
                 double *gscale, int *err, cudaStream_t stream) {
-    if (n_sel > 0) {
+    if (g.order) {
+        const double *m = reinterpret_cast<const double *>(model);
+        const int st = launch_dense_grid<CT, GRAD>(g, n_sel, size, m, m + 1, 2, vscale, bg_sum, dia,
+                                                   sx, sy, scale, n_frames, out, gre, gim, gdia,
+                                                   gsx, gsy, gscale, stream);
+        if (st != RSPI_OK) return st;
+    } else if (n_sel > 0) {
         const dim3 grid((unsigned)((n_sel + 255) / 256),
                         (unsigned)((n_frames + EN_FRAMES - 1) / EN_FRAMES));
         k_emc_nll_msum<CT, GRAD><<<grid, 256, 0, stream>>>(model, size, bg, sel_pix, n_sel, dia,
@@ -287,11 +294,12 @@ void emc_launch(const double2 *model, int size, const double *bg, const int *sel
     k_emc_nll_photons<CT, GRAD><<<rspi_blocks(n_frames * 32, 256), 256, 0, stream>>>(
         ones, multi, oacc, macc, po, pm, cm, n_frames, model, size, bg, pix2sel, rot_cs, dia, sx,
         sy, scale, out, gre, gim, gdia, gsx, gsy, gscale, err);
+    RSPI_RETURN_LAUNCH();
 }
 
 }  // namespace
 
-extern "C" int rspi_emc_nll(int precision, int want_grad, const double *model, long long size,
+static int emc_nll_entry(const GridTables &g, double bg_sum, int precision, int want_grad, const double *model, long long size,
                             const double *bg, const int *sel_pix, long long n_sel,
                             const int *pix2sel, const int *ones, const int *multi,
                             const long long *ones_accum, const long long *multi_accum,
@@ -318,14 +326,52 @@ extern "C" int rspi_emc_nll(int precision, int want_grad, const double *model, l
         cudaMemsetAsync(gscale, 0, sizeof(double) * n_frames, stream);
     }
     const double2 *m = reinterpret_cast<const double2 *>(model);
-#define RSPI_ENLL(CT, G)                                                                       \
-    emc_launch<CT, G>(m, (int)size, bg, sel_pix, n_sel, pix2sel, ones, multi, ones_accum,       \
+#define RSPI_ENLL(CT, G)                                                                           \
+    emc_launch<CT, G>(g, bg_sum, m, (int)size, bg, sel_pix, n_sel, pix2sel, ones, multi, ones_accum, \
                       multi_accum, place_ones, place_multi, count_multi, n_frames, rot_cs, dia, \
                       sx, sy, scale, vscale, nll, gre, gim, gdia, gsx, gsy, gscale, err, stream)
-    if (precision == 1 && want_grad) RSPI_ENLL(double, true);
-    else if (precision == 1) RSPI_ENLL(double, false);
-    else if (want_grad) RSPI_ENLL(float, true);
-    else RSPI_ENLL(float, false);
+    if (precision == 1 && want_grad) return RSPI_ENLL(double, true);
+    if (precision == 1) return RSPI_ENLL(double, false);
+    if (want_grad) return RSPI_ENLL(float, true);
+    return RSPI_ENLL(float, false);
 #undef RSPI_ENLL
-    RSPI_RETURN_LAUNCH();
+}
+
+extern "C" int rspi_emc_nll(int precision, int want_grad, const double *model, long long size,
+                            const double *bg, const int *sel_pix, long long n_sel,
+                            const int *pix2sel, const int *ones, const int *multi,
+                            const long long *ones_accum, const long long *multi_accum,
+                            const int *place_ones, const int *place_multi,
+                            const int *count_multi, long long n_frames, const double *rot_cs,
+                            const double *dia, const double *sx, const double *sy,
+                            const double *scale, double vscale, double *nll, double *gre,
+                            double *gim, double *gdia, double *gsx, double *gsy, double *gscale,
+                            int *err, cudaStream_t stream) {
+    const GridTables none{nullptr, nullptr, nullptr, nullptr, 0};
+    return emc_nll_entry(none, 0.,
+                         precision, want_grad, model, size, bg, sel_pix, n_sel, pix2sel,
+                         ones, multi, ones_accum, multi_accum, place_ones, place_multi,
+                         count_multi, n_frames, rot_cs, dia, sx, sy, scale, vscale, nll,
+                         gre, gim, gdia, gsx, gsy, gscale, err, stream);
+}
+
+extern "C" int rspi_emc_nll_grid(int precision, int want_grad, const double *model, long long size,
+                                 const double *bg, const int *sel_pix, long long n_sel, const int
+                                 *order, const int *xy, const int *rad_id, const double *rad_q, int
+                                 tile_rads, double bg_sum, const int *pix2sel, const int *ones,
+                                 const int *multi, const long long *ones_accum, const long long
+                                 *multi_accum, const int *place_ones, const int *place_multi, const
+                                 int *count_multi, long long n_frames, const double *rot_cs, const
+                                 double *dia, const double *sx, const double *sy, const double
+                                 *scale, double vscale, double *nll, double *gre, double *gim,
+                                 double *gdia, double *gsx, double *gsy, double *gscale, int *err,
+                                 cudaStream_t stream) {
+    if (!grid_tables_ok(precision, size, n_sel, order, xy, rad_id, rad_q, tile_rads))
+        return RSPI_ERR_ARG;
+    const GridTables g{order, xy, rad_id, rad_q, tile_rads};
+    return emc_nll_entry(g, bg_sum,
+                         precision, want_grad, model, size, bg, sel_pix, n_sel, pix2sel,
+                         ones, multi, ones_accum, multi_accum, place_ones, place_multi,
+                         count_multi, n_frames, rot_cs, dia, sx, sy, scale, vscale, nll,
+                         gre, gim, gdia, gsx, gsy, gscale, err, stream);
 }

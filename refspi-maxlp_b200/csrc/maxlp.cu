@@ -51,20 +51,18 @@ __global__ void k_frame_params(const int *__restrict__ rmax, long long n, long l
 __device__ __forceinline__ void scatter_photon(int ux, int uy, int cnt, double c, double s,
                                                int size, const int *__restrict__ mask_idx,
                                                long long n_ref, int st, int *__restrict__ hist) {
-    const double c0 = (double)(size / 2);
-    const double vx = (double)ux - c0, vy = (double)uy - c0;
-    const int bx = (int)rint(c * vx + s * vy + c0);
-    const int by = (int)rint(-s * vx + c * vy + c0);
-    for (int ax = -1; ax <= 1; ++ax)
-        for (int ay = -1; ay <= 1; ++ay) {
-            const int tx = bx + ax, ty = by + ay;
-            if (tx < 0 || ty < 0 || tx >= size || ty >= size) continue;
-            const int m = mask_idx[tx * size + ty];
-            if (m < 0) continue;
-            int ox, oy;
-            forward_pixel(tx, ty, c, s, size, ox, oy);
-            if (ox == ux && oy == uy) atomicAdd(&hist[(long long)m * n_ref + st], cnt);
-        }
+    int bx, by;
+    for (unsigned near = near_pixels(ux, uy, c, s, (double)(size / 2), bx, by); near;
+         near &= near - 1) {
+        const int k = __ffs(near) - 1;
+        const int tx = bx + k / 3 - 1, ty = by + k % 3 - 1;
+        if (tx < 0 || ty < 0 || tx >= size || ty >= size) continue;
+        const int m = mask_idx[tx * size + ty];
+        if (m < 0) continue;
+        int ox, oy;
+        forward_pixel(tx, ty, c, s, size, ox, oy);
+        if (ox == ux && oy == uy) atomicAdd(&hist[(long long)m * n_ref + st], cnt);
+    }
 }
 
 __global__ void __launch_bounds__(256)

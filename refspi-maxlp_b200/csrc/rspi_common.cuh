@@ -73,14 +73,42 @@ __device__ __forceinline__ double rot_log_value(const double *__restrict__ w, in
 
 // Detector pixel of model pixel (tx, ty) for a frame with rotation (c, s):
 // maxLP.py:250-252, x' = c qx + (-s) qy, y' = s qx + c qy, rint(x' size + size//2).
-__device__ __forceinline__ void forward_pixel(int tx, int ty, double c, double s, int size,
-                                              int &ox, int &oy) {
+__device__ __forceinline__ void forward_q(double qx, double qy, double c, double s, int size,
+                                          int &ox, int &oy) {
     const double ds = (double)size, c0 = (double)(size / 2);
-    const double qx = ((double)tx - c0) / ds, qy = ((double)ty - c0) / ds;
     const double xr = xadd(xmul(c, qx), xmul(-s, qy));
     const double yr = xadd(xmul(s, qx), xmul(c, qy));
     ox = (int)rint(xadd(xmul(xr, ds), c0));
     oy = (int)rint(xadd(xmul(yr, ds), c0));
+}
+__device__ __forceinline__ void forward_pixel(int tx, int ty, double c, double s, int size,
+                                              int &ox, int &oy) {
+    const double ds = (double)size, c0 = (double)(size / 2);
+    forward_q(((double)tx - c0) / ds, ((double)ty - c0) / ds, c, s, size, ox, oy);
+}
+
+// The pixels of the 3 x 3 neighbourhood of (bx, by), the rounded inverse
+// image of detector pixel (ux, uy), that forward_pixel can map onto it (bit
+// 3 (ax + 1) + ay + 1 for (bx + ax, by + ay)): those whose forward image lies
+// within half a pixel of (ux, uy), tested in FP32 with a margin of 1e-3 (its
+// error is below 1e-5).  About one of nine passes; each still takes the exact
+// test, whose two FP64 divisions made it most of the photon kernels' time.
+__device__ __forceinline__ unsigned near_pixels(int ux, int uy, double c, double s, double c0,
+                                                int &bx, int &by) {
+    const double vx = (double)ux - c0, vy = (double)uy - c0;
+    const double ix = c * vx + s * vy + c0, iy = -s * vx + c * vy + c0;
+    bx = (int)rint(ix);
+    by = (int)rint(iy);
+    const float ox = (float)((double)bx - ix), oy = (float)((double)by - iy);
+    const float cf = (float)c, sf = (float)s;
+    unsigned mask = 0;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        const float ex = ox + (float)(k / 3 - 1), ey = oy + (float)(k % 3 - 1);
+        if (fabsf(cf * ex - sf * ey) <= 0.501f && fabsf(sf * ex + cf * ey) <= 0.501f)
+            mask |= 1u << k;
+    }
+    return mask;
 }
 
 template <class T>

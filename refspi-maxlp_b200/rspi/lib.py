@@ -61,9 +61,13 @@ SIGNATURES = {
     'rspi_screen_candidates_noalloc': (I, [P, L, L, P, P, P, P, P, D, P, P, P, P, L, P, P, P,
                                            P]),
     'rspi_nll': (I, [I, I] + [P] * 7 + [L, P, L, P, L] + [P] * 18),
+    'rspi_nll_grid': (I, [I, I] + [P] * 7 + [L, P, L, P, L] + [P] * 4 + [I] + [P] * 18),
+    'rspi_nll_grid_tile': (I, [I, L]),
     'rspi_entries16_check': (I, [P, L, P, P]),
     'rspi_emc_nll': (I, [I, I, P, L, P, P, L, P, P, P, P, P, P, P, P, L, P, P, P, P, P, D, P,
                          P, P, P, P, P, P, P, P]),
+    'rspi_emc_nll_grid': (I, [I, I, P, L, P, P, L] + [P] * 4 + [I, D] + [P] * 8 + [L] + [P] * 5 +
+                          [D] + [P] * 9),
     'rspi_cdft2': (I, [P, P, P, L, I, P]),
     'rspi_phase_support': (I, [P, L, D, D, D, I, D, P, P, P]),
     'rspi_phase_proj_fourier': (I, [P, P, P, P, L, P]),
@@ -143,11 +147,11 @@ KERNELS_PER_CALL = {
     'rspi_screen_loglike7': 1, 'rspi_quad4_part_sums_floats': 0,
     'rspi_mean': 1, 'rspi_ll16_entry_rows': 1, 'rspi_ll16_entry_fill': 1, 'rspi_screen_candidates': 3, 'rspi_rescore': 5,
     'rspi_loglike_stream': 1, 'rspi_posterior_pairs': 3,
-    'rspi_entries16_check': 1, 'rspi_emc_nll': 2, 'rspi_cdft2': 2, 'rspi_phase_support': 5,
+    'rspi_entries16_check': 1, 'rspi_emc_nll': 2, 'rspi_emc_nll_grid': 2, 'rspi_cdft2': 2, 'rspi_phase_support': 5,
     'rspi_phase_proj_fourier': 1, 'rspi_phase_proj_real': 4, 'rspi_sets_counts': 1, 'rspi_sets_group': 1, 'rspi_sets_steps': 1,
     'rspi_sets_fill': 1, 'rspi_rot_log_slices_sets': 1, 'rspi_holo_quads32': 1, 'rspi_sets_part_sums_floats': 0,
     'rspi_screen_loglike_sets': 1, 'rspi_frame_max_finalize': 1,
-    'rspi_screen_candidates_cols': 4, 'rspi_rescore_cols': 5, 'rspi_nll': 2, 'rspi_screen_candidates_noalloc': 3, 'rspi_merge_coverage': 1, 'rspi_merge': 2,
+    'rspi_screen_candidates_cols': 4, 'rspi_rescore_cols': 5, 'rspi_nll': 2, 'rspi_nll_grid': 2, 'rspi_screen_candidates_noalloc': 3, 'rspi_merge_coverage': 1, 'rspi_merge': 2,
     'rspi_dense_frames': 1, 'rspi_rot_log_split': 1, 'rspi_dense_loglike': 1,
     'rspi_maxlp_grid': 2, 'rspi_dense_frames_u8': 1, 'rspi_rot_log_fixed': 1,
     'rspi_dense_loglike_i8': 1, 'rspi_sets_entries_check': 1, 'rspi_sim_views': 1, 'rspi_sim_counts': 1,
