@@ -428,6 +428,20 @@ int rspi_rescore(const int *cand_d, const int *cand_r, const long long *cand_off
                  const double *noncand, double *maxll, int *rmax, double *logz,
                  double *row_scratch, long long scratch_rows, cudaStream_t stream);
 
+/* rspi_rescore for densely stored frames (n_data x size^2 counts): each row's
+ * FP64 rotated slice is built a tile of columns at a time and multiplied with
+ * its candidates' counts there, instead of walking their sparse entries (the
+ * sums differ from rspi_rescore's by their FP64 rounding). */
+int rspi_rescore_dense(const int *cand_d, const int *cand_r, const long long *cand_off,
+                       long long n_data, long long capacity, long long n_rows,
+                       const unsigned short *frames, const double *holo, long long num_rot,
+                       const double *rot_cs, long long size, const double *bg,
+                       const int *sel_pix, long long n_sel, const double *init,
+                       const double *scales, int *row_cnt, long long *row_cand_off,
+                       int *row_cand, double *cand_ll, float *ll32, const double *max32,
+                       const double *noncand, double *maxll, int *rmax, double *logz,
+                       cudaStream_t stream);
+
 /* rspi_rescore for a likelihood matrix with n_cols columns in which frame d
  * is column col_of_frame[d]. */
 int rspi_rescore_cols(const int *cand_d, const int *cand_r, const long long *cand_off,

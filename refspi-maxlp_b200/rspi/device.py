@@ -826,6 +826,14 @@ class EStep:
                     continue
                 self.n_candidates = total
             break
+        if self.form == 'dense':
+            call('rspi_rescore_dense', ptr(self.cand_d), ptr(self.cand_r), ptr(self.cand_off), n,
+                 self.capacity, self.n_rows, ptr(self.ph.frames), ptr(self.holo), self.num_rot,
+                 ptr(self.rot_cs), self.size, ptr(self.bg), ptr(self.sel_pix), self.n_sel,
+                 ptr(self.init), ptr(self.ph.scales), ptr(self.row_cnt), ptr(self.row_cand_off),
+                 ptr(self.row_cand), ptr(self.cand_ll), ptr(self.prob), ptr(self.max32),
+                 ptr(self.noncand), ptr(self.maxll), ptr(self.rmax), ptr(self.logz), s)
+            return self.maxll, self.rmax, self.logz
         head = (ptr(self.cand_d), ptr(self.cand_r), ptr(self.cand_off), n, self.capacity,
                 self.n_rows, ptr(self.holo), self.num_rot, ptr(self.rot_cs), self.size,
                 ptr(self.bg), ptr(self.sel_pix), self.n_sel, self.p_pad, ptr(self.init),
