@@ -341,7 +341,7 @@ class MaxLPhaser():
         inv, supp = self._bytes(self.minvmask), self._bytes(self.minvsuppmask)
         call('rspi_phase_refine', ptr(fconv), ptr(inv), ptr(supp), ptr(out), ptr(self._work()),
              self.size, int(n_dm), int(n_er), cur_stream())
-        rlib.launch_count += 5 * (int(n_dm) + int(n_er))
+        rlib.launch_count += 2 * (int(n_dm) + int(n_er)) + 1
         return out
 
     def er(self, fconv, x):
