@@ -21,33 +21,58 @@ __device__ __forceinline__ double holo_value(const double2 m, double dx, double 
     const double phase = xmul(2. * PI, xadd(xmul(dx, sx), xmul(dy, sy))) / size;
     double s = xmul(xmul(sqrt(xadd(xmul(dx, dx), xmul(dy, dy))), PI), dia) / size;
     if (s == 0.) s = 1.e-5;
-    const double sphere = (1.0 * xsub(sin(s), xmul(s, cos(s)))) / xmul(xmul(s, s), s);
-    const double re = xadd(xmul(cos(phase), sphere), m.x);
-    const double im = xadd(xmul(sin(phase), sphere), m.y);
+    double sn, cs;
+    sincos(s, &sn, &cs);
+    const double sphere = (1.0 * xsub(sn, xmul(s, cs))) / xmul(xmul(s, s), s);
+    sincos(phase, &sn, &cs);
+    const double re = xadd(xmul(cs, sphere), m.x);
+    const double im = xadd(xmul(sn, sphere), m.y);
     return xadd(xadd(xmul(re, re), xmul(im, im)), bg);
 }
 
+// One CTA per HOLO_TILE pixels of a state: about 250 FP64 operations a pixel
+// bound it, so the pixels of few states have to fill the GPU too (a CTA per
+// state left 121 of 148 SMs idle at 27 states: 0.37 ms, now 0.02 at
+// 255^2; 0.20, now 0.03, at 75 states of 185^2).
+constexpr int HOLO_TILE = 4 * HOLO_THREADS;
+
 __global__ void __launch_bounds__(HOLO_THREADS)
 k_holo(const double2 *__restrict__ model, const double *__restrict__ shiftx,
-       const double *__restrict__ shifty, const double *__restrict__ sphere_dia, long long size,
-       const double *__restrict__ bg, const int *__restrict__ sel_pix, long long n_sel,
-       double *__restrict__ holo, double *__restrict__ msum) {
-    __shared__ double scratch[32];
-    const long long s0 = blockIdx.x;
-    const long long npix = size * size;
+       const double *__restrict__ shifty, const double *__restrict__ sphere_dia, int size,
+       int tiles, const double *__restrict__ bg, double *__restrict__ holo) {
+    const long long s0 = blockIdx.x / (unsigned)tiles;
+    const int p0 = (int)(blockIdx.x % (unsigned)tiles) * HOLO_TILE;
+    const int npix = size * size;
     const double sx = shiftx[s0], sy = shifty[s0], dia = sphere_dia[s0];
     const double cen = floor(size / 2.);
     const double dsize = (double)size;
     double *w = holo + s0 * npix;
-    for (long long p = threadIdx.x; p < npix; p += blockDim.x) {
-        const long long x = p / size, y = p - x * size;
+    const int p1 = min(npix, p0 + HOLO_TILE);
+    for (int p = p0 + threadIdx.x; p < p1; p += HOLO_THREADS) {
+        const int x = p / size, y = p - x * size;
         w[p] = holo_value(model[p], (double)x - cen, (double)y - cen, sx, sy, dia, dsize, bg[p]);
     }
-    __syncthreads();
+}
+
+// Masked sum of one state's slice per CTA: thread t sums the likelihood
+// pixels t, t + 256, ... in order, eight loads in flight.
+__global__ void __launch_bounds__(HOLO_THREADS)
+k_holo_msum(const double *__restrict__ holo, long long npix, const int *__restrict__ sel_pix,
+            long long n_sel, double *__restrict__ msum) {
+    __shared__ double scratch[32];
+    const double *w = holo + blockIdx.x * npix;
     double acc = 0.;
-    for (long long c = threadIdx.x; c < n_sel; c += blockDim.x) acc += w[sel_pix[c]];
+    long long c = threadIdx.x;
+    for (; c + 7 * HOLO_THREADS < n_sel; c += 8 * HOLO_THREADS) {
+        double v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = w[sel_pix[c + k * HOLO_THREADS]];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) acc += v[k];
+    }
+    for (; c < n_sel; c += HOLO_THREADS) acc += w[sel_pix[c]];
     acc = block_sum(acc, scratch);
-    if (threadIdx.x == 0) msum[s0] = acc;
+    if (threadIdx.x == 0) msum[blockIdx.x] = acc;
 }
 
 // EMC.sphere and EMC.ramp of one state (emc.py:244-254): with integer-centred
@@ -98,7 +123,7 @@ k_vscale_init(const double *__restrict__ msum, long long n_states0,
 // the same FP64 interpolation and log as rot_log_value (identical values)
 // and one store.  With PAIRS the four neighbours come as two 16-byte loads
 // from the paired copy hp[p] = (w[p], w[p + 1]) of the holographic slices.
-constexpr int RL_STATES = 8;
+constexpr int RL_STATES = 8;   // 4, 5 and 16 measured slower at 405, 245 and 225 states
 
 // hp[i] = (holo[i], holo[i + 1]) over the whole state-major array (0 past
 // its end); only pairs of a pixel and its right neighbour in the same row
@@ -485,9 +510,12 @@ extern "C" int rspi_holo_slices(const double *model, const double *shiftx, const
                                 double *holo, double *msum, cudaStream_t stream) {
     if (n_states0 <= 0 || size <= 1 || n_sel < 0 || !model || !holo || !msum || !bg)
         return RSPI_ERR_ARG;
-    if (n_states0 > 0x7fffffffLL) return RSPI_ERR_ARG;
-    k_holo<<<(unsigned)n_states0, HOLO_THREADS, 0, stream>>>(
-        (const double2 *)model, shiftx, shifty, sphere_dia, size, bg, sel_pix, n_sel, holo, msum);
+    const long long tiles = (size * size + HOLO_TILE - 1) / HOLO_TILE;
+    if (size > 46340 || n_states0 > 0x7fffffffLL / tiles) return RSPI_ERR_ARG;
+    k_holo<<<(unsigned)(n_states0 * tiles), HOLO_THREADS, 0, stream>>>(
+        (const double2 *)model, shiftx, shifty, sphere_dia, (int)size, (int)tiles, bg, holo);
+    k_holo_msum<<<(unsigned)n_states0, HOLO_THREADS, 0, stream>>>(holo, size * size, sel_pix, n_sel,
+                                                                 msum);
     RSPI_RETURN_LAUNCH();
 }
 

@@ -137,7 +137,7 @@ def check(code, what):
 # kernels each entry point launches (memsets are not counted)
 KERNELS_PER_CALL = {
     'rspi_photon_offsets': 4, 'rspi_powder': 2, 'rspi_ll_entry_rows': 1, 'rspi_scan_rows': 1,
-    'rspi_ll_entry_fill': 1, 'rspi_holo_slices': 1, 'rspi_vscale_init': 1,
+    'rspi_ll_entry_fill': 1, 'rspi_holo_slices': 2, 'rspi_vscale_init': 1,
     'rspi_rot_log_slices': 1, 'rspi_holo_pairs': 1, 'rspi_rot_log_slices_pairs': 1,
     'rspi_loglike': 1, 'rspi_frame_reduce': 1,
     'rspi_maxlp_frame_params': 1, 'rspi_maxlp_histogram': 1, 'rspi_maxlp_pixel_map': 3,
