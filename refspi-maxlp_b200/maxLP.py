@@ -26,6 +26,19 @@ from rspi import lib as rlib  # noqa: E402
 from rspi.lib import call  # noqa: E402
 
 
+def _unique_rows(rows):
+    '''np.unique(rows, axis=0, return_inverse=True): the rows in lexicographic
+    order and each row's place, from a sort per column (np.unique compares the
+    rows as records: 0.6 ms of a 1.6 ms call for 1,000 frames, 0.1 ms here).'''
+    order = np.lexsort(rows.T[::-1])
+    first = np.ones(order.size, dtype=bool)
+    srt = rows[order]
+    first[1:] = np.any(srt[1:] != srt[:-1], axis=1)
+    place = np.empty(order.size, dtype=np.int64)
+    place[order] = np.cumsum(first) - 1
+    return srt[first], place
+
+
 class MaxLPhaser():
     '''Reconstruction of object from holographic data using maximum likelihood and pattern search'''
     def __init__(self, data_fname, size=185, num_data=-1, dataset=None, device=None,
@@ -267,11 +280,10 @@ class MaxLPhaser():
         self.diams = dia
         self.ang = ang
         self._ftab = None   # the per-pixel API's frame tables follow these
-        triples = np.stack([sx, sy, dia], axis=1)
-        ref, fstate = np.unique(triples, axis=0, return_inverse=True)
+        ref, fstate = _unique_rows(np.stack([sx, sy, dia], axis=1))
         dev = self.device
         ref_params = torch.from_numpy(np.ascontiguousarray(ref)).to(dev)
-        fstate = modes.astype(np.int64) * ref.shape[0] + fstate.ravel()
+        fstate = modes.astype(np.int64) * ref.shape[0] + fstate
         fstate_t = torch.from_numpy(fstate.astype('i4')).to(dev)
         frot_t = torch.arange(self.num_data, dtype=torch.int32, device=dev)
         nstate = torch.from_numpy(np.bincount(fstate, minlength=nm * ref.shape[0]).astype('i4')).to(dev)
