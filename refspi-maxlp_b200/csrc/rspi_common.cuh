@@ -216,3 +216,33 @@ static inline unsigned rspi_blocks(long long work, int threads, int cap_per_sm =
 // Exclusive scan of n int32 counts into off[0..n] (the total at [n]); one or
 // three launches (scan.cu).
 int rspi_scan_i32(const int *cnt, long long n, long long *off, cudaStream_t stream);
+
+// CTAs (of a cluster, along y) that share the rows of a 32-column block in
+// the passes over a likelihood matrix: with a CTA per block of columns, a few
+// thousand frames leave most SMs without one (32 of 148 at 1,000 frames).
+// Up to 8, while the blocks do not fill the GPU and every CTA keeps at least
+// 512 rows.
+static inline unsigned rspi_row_ctas(long long blocks, long long n_rows) {
+    unsigned n = 1;
+    while (n < 8 && blocks * n < rspi_sm_count() && n_rows >= 1024LL * n) n *= 2;
+    return n;
+}
+
+// Launches `kernel` on grid (blocks, n) with clusters of n CTAs along y.
+template <class... P, class... A>
+static inline int rspi_launch_rows(void (*kernel)(P...), long long blocks, unsigned n, dim3 block,
+                                   cudaStream_t stream, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks, n);
+    cfg.blockDim = block;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = n;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...) == cudaSuccess ? RSPI_OK
+                                                                                    : RSPI_ERR_CUDA;
+}
