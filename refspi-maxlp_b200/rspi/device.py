@@ -861,6 +861,8 @@ class Merge:
     """Posterior-weighted merge into per-(shift, diameter) intensities (a10)."""
 
     def __init__(self, estep, p_min=1.e-6, pairs_per_frame=16):
+        if estep.form == 'dense' and not estep.rescore:
+            raise ValueError('the merge needs the candidates of dense_rescore')
         self.es = estep
         self.p_min = float(p_min)
         dev = estep.device
@@ -872,7 +874,11 @@ class Merge:
         self.w = torch.empty(n0 * r, dtype=_f64, device=dev)
         self.intens = torch.empty((n0, npix), dtype=_f64, device=dev)
         n = estep.ph.num_data
-        if estep.form == 'fp64':
+        if estep.form != 'fp64':
+            # an unrotated image per CTA of the row-grouped scatter, two per SM
+            sms = torch.cuda.get_device_properties(dev).multi_processor_count
+            self.images = torch.empty((2 * sms, npix), dtype=_f64, device=dev)
+        else:
             self.cnt_part = torch.empty(n * 32, dtype=_i32, device=dev)
             self.cnt = torch.empty(n, dtype=_i32, device=dev)
             self.off = torch.empty(n + 1, dtype=_i64, device=dev)
@@ -899,9 +905,16 @@ class Merge:
                     break
                 ph.err.t.zero_()
                 self._alloc(int(total * 1.25) + 1024)
-            pd, pr, pll, tot, cap = self.pd, self.pr, self.pll, self.off[n:], self.capacity
         else:
-            pd, pr, pll, tot, cap = es.cand_d, es.cand_r, es.cand_ll, es.cand_off[n:], es.capacity
+            # the rescoring left the candidates grouped by likelihood row
+            call('rspi_merge_rows', ptr(es.cand_d), ptr(es.cand_ll), ptr(es.row_cand_off),
+                 ptr(es.row_cand), ptr(es.logz), self.p_min, ptr(ph.scales), ptr(ph.ones),
+                 ptr(ph.multi), ptr(ph.ones_accum), ptr(ph.multi_accum), ptr(ph.place_ones),
+                 ptr(ph.place_multi), ptr(ph.count_multi), es.n_states0, es.num_rot,
+                 ptr(es.rot_cs), es.size, ptr(self.cov), ptr(self.num), ptr(self.den),
+                 ptr(self.w), ptr(self.intens), ptr(self.images), self.images.shape[0], s)
+            return self.intens
+        pd, pr, pll, tot, cap = self.pd, self.pr, self.pll, self.off[n:], self.capacity
         call('rspi_merge', ptr(pd), ptr(pr), ptr(pll), ptr(tot), cap, ptr(es.logz), self.p_min,
              ptr(ph.scales), ptr(ph.ones), ptr(ph.multi), ptr(ph.ones_accum), ptr(ph.multi_accum),
              ptr(ph.place_ones), ptr(ph.place_multi), ptr(ph.count_multi), es.n_states0,
