@@ -32,25 +32,30 @@ def _orbit_tables(size, prec, pixels, rows, qrad, t):
     if tile < 0 or pixels.size == 0:
         return None
     c = size // 2
-    x, y = pixels // size - c, pixels % size - c
+    x, y = np.divmod(pixels.astype(np.int64), size)
+    x -= c
+    y -= c
     rep = np.flatnonzero((x >= 1) & (y >= 0))
-    rep = rep[np.argsort(x[rep] ** 2 + y[rep] ** 2, kind='stable')]
-    _, first, rad = np.unique(x[rep] ** 2 + y[rep] ** 2, return_index=True, return_inverse=True)
+    r2 = x[rep] ** 2 + y[rep] ** 2
+    by_r2 = np.argsort(r2, kind='stable')
+    rep, r2 = rep[by_r2], r2[by_r2]
+    new = np.ones(rep.size, dtype=bool)
+    new[1:] = r2[1:] != r2[:-1]
+    rad, q_rad = np.cumsum(new) - 1, qrad[rep[new]]
     # groups of neighbouring radii, within them by row: lanes then read the
     # phase tables side by side
-    by = np.lexsort((y[rep], x[rep], np.arange(rep.size) // tile))
-    q_rad = qrad[rep][first]
-    rep, rad = rep[by], rad.ravel()[by]
+    group = np.arange(rep.size) // tile
+    spans = rad[np.minimum(np.arange(tile, rep.size + tile, tile), rep.size) - 1] - rad[::tile] + 1
+    by = np.argsort((group * (size + 1) + x[rep]) * (size + 1) + y[rep])
+    rep, rad = rep[by], rad[by]
     xr, yr = x[rep], y[rep]
     row = np.full((size + 1,) * 2, -1, dtype='i4')   # + 1: coordinates -c .. c
     row[x, y] = rows
     order = np.stack([row[xr, yr], row[-yr, xr], row[-xr, -yr], row[yr, -xr]], axis=1)
-    if order.size != pixels.size or (order.size and order.min() < 0):
+    if order.size != pixels.size or order.min() < 0:
         return None
-    spans = [rad[i:i + tile].max() - rad[i:i + tile].min() + 1 for i in range(0, rad.size, tile)]
     i32 = torch.int32
-    return (t(order, i32), t((xr << 16) | yr, i32), t(rad, i32), t(q_rad, _f64),
-            int(max(spans, default=1)))
+    return (t(order, i32), t((xr << 16) | yr, i32), t(rad, i32), t(q_rad, _f64), int(spans.max()))
 
 
 class NLLProblem:
