@@ -244,12 +244,19 @@ int rspi_screen_loglike7(const float *lslices, long long p_row, long long num_ro
  * into n_parts (1-4) parts of part_w columns (part_w % 8 == 0,
  * n_parts * part_w >= p_zero), each staged in shared memory as four FP32
  * rows per column with 8 zero columns after it.
- * rspi_sets_counts: counts[d * 32 + 8 h + c] = frame d's photons in part h of
- * local column class c (local column mod 8), from the 16-bit entries of
- * rspi_ll16_entry_fill (p_zero = their zero column).
+ * A set entry is a local column (bits 0-13) with the logarithm of its
+ * photons, 1, 2, 4 or 8 (bits 14-15).
+ * rspi_sets_counts32: counts[d * 32 + 8 h + c] = frame d's entries in part h
+ * of local column class c (local column mod 8): a pixel of k photons takes
+ * floor(k / 8) entries of 8 and one per binary digit of k mod 8; from the
+ * packed entries of rspi_ll_entry_fill (column << 16 | count; columns from
+ * p_zero on, a multiple of 32, are not photons).  part_w <= 16376.
+ * rspi_sets_counts: the same with every photon an entry of its own, from the
+ * 16-bit entries of rspi_ll16_entry_fill (p_zero = their zero column); the
+ * forms of the two calls go together (counts32 with fill32).
  * rspi_sets_group: set_frames[32 * ceil(n_data / 32)] from `order` (the
- * frames by decreasing photon count, a permutation of [0, n_data)) and
- * rspi_sets_counts' counts: per window of 256 consecutive ranks, quarters of
+ * frames by decreasing entry count, a permutation of [0, n_data)) and
+ * the counts: per window of 256 consecutive ranks, quarters of
  * eight frames built greedily (each from the longest frame left, adding the
  * frame that keeps sum over parts of max(largest frame, largest class total)
  * smallest), then up to `sweeps` sweeps over every pair of the window's
@@ -265,14 +272,14 @@ int rspi_screen_loglike7(const float *lslices, long long p_row, long long num_ro
  * eight frames) (Koenig's edge-colouring bound); groups[h * n_sets + s] =
  * the largest of the four.  The caller scans the groups part-major into
  * group_off[n_parts*n_sets + 1].
- * rspi_sets_fill: group_off[last] * 128 16-bit entries (8-byte aligned,
- * prefilled by the caller with any value <= part_w + 7): entry
- * ((g * 32 + lane) * 4 + k) is the local column the lane reads at step
+ * rspi_sets_fill32, rspi_sets_fill: group_off[last] * 128 16-bit entries
+ * (8-byte aligned, prefilled by the caller with any value <= part_w + 7):
+ * entry ((g * 32 + lane) * 4 + k) is what the lane reads at step
  * 4 (g - g0) + k of its (set, part) range [g0, g1).  A quarter warp runs
  * its own D_q steps (max of its largest frame count and largest class
  * total), in each of which its eight lanes read eight distinct classes (a
  * Birkhoff-von Neumann decomposition of the count matrix padded to a
- * regular one), real photons first, the zero column part_w + class
+ * regular one), real entries first, the zero column part_w + class
  * otherwise; from step D_q on each lane holds the zero column of its own
  * class (rspi_screen_loglike_sets skips those groups of the quarter warp
  * when given quarter_groups).  A schedule that cannot be built sets
@@ -280,6 +287,9 @@ int rspi_screen_loglike7(const float *lslices, long long p_row, long long num_ro
 int rspi_sets_counts(const unsigned short *entries16, const long long *row_off16,
                      long long n_data, int p_zero, int n_parts, int part_w, int *counts,
                      cudaStream_t stream);
+int rspi_sets_counts32(const unsigned int *entries32, const long long *row_off32,
+                       long long n_data, int p_zero, int n_parts, int part_w, int *counts,
+                       cudaStream_t stream);
 int rspi_sets_group(const int *counts, const int *order, long long n_data, int n_parts,
                     int sweeps, int *set_frames, int *err, cudaStream_t stream);
 int rspi_sets_steps(const int *counts, const int *set_frames, long long n_sets, int n_parts,
@@ -288,6 +298,10 @@ int rspi_sets_fill(const unsigned short *entries16, const long long *row_off16, 
                    int n_parts, int part_w, const int *counts, const int *set_frames,
                    long long n_sets, const long long *group_off, unsigned short *entries,
                    int *err, cudaStream_t stream);
+int rspi_sets_fill32(const unsigned int *entries32, const long long *row_off32, int p_zero,
+                     int n_parts, int part_w, const int *counts, const int *set_frames,
+                     long long n_sets, const long long *group_off, unsigned short *entries,
+                     int *err, cudaStream_t stream);
 
 /* Rotated log-slices in the layout of rspi_screen_loglike_sets: rows taken
  * four at a time from row_begin, columns cut into parts:
@@ -314,8 +328,9 @@ int rspi_rot_log_slices_sets(const double *holo_pairs, const float *holo_quads32
 /* FP32 screening likelihood of rows [row_begin, row_end) from those slices
  * (one bulk copy per tile part into shared memory) and the set entries: lane l
  * of set s sums its frame's photons in the four rows (two alternating FP32
- * accumulators over the groups, each group's four photons as a depth-two
- * tree: at most ceil(G/2) + 3 roundings per value and part, G = the set's
+ * accumulators over the groups, each group's four entries, taken exactly
+ * times an eighth of their counts, as a depth-two tree; the sum times 8 at
+ * the end: at most ceil(G/2) + 3 roundings per value and part, G = the set's
  * groups in the part); the parts are added in FP64 before the final
  * rounding, the running sum of parts before the last kept in the SM's
  * tensor memory for the first 512 sets (each CTA allocates all 512 TMEM
@@ -328,15 +343,39 @@ int rspi_rot_log_slices_sets(const double *holo_pairs, const float *holo_quads32
  * ll[(r - row_begin) * ll_stride + c] (ll_stride >= n_sets * 32), and
  * frame_max[c] (zero before the first launch of a pass) takes the unsigned
  * maximum of an order-preserving (value, row) key, read and reset by
- * rspi_frame_max_finalize.  A bulk copy that does not complete within 1 s
- * sets *err = RSPI_ERR_TIMEOUT and the kernel returns.  Requires every entry
- * <= part_w + 7 (check with rspi_sets_entries_check). */
+ * rspi_frame_max_finalize.  rspi_screen_loglike_sets takes the entries of
+ * rspi_sets_fill; rspi_screen_loglike_items those of rspi_sets_fill32 as well
+ * (counted != 0) and, with items != NULL, cuts long sets into pieces: items
+ * [item_off[h * Q + q], item_off[h * Q + q + 1]) are those of part h, queue q
+ * (Q = 4 queues with several parts, set s in queue s % 4, else 1), each eight
+ * ints (16-byte aligned table): the set, its first group, its groups, base |
+ * piece << 16 | pieces << 24 (pieces 1: the whole set; more, at most 127,
+ * only for sets < 64: the pieces cover the set, piece i adding to slot
+ * base + i < seg_slots of the part), and the groups of each quarter warp.
+ * seg_sums holds 128 * seg_slots * seg_ctas floats (16-byte aligned; at most
+ * seg_ctas CTAs run).  A split set's pieces are added in FP64 in their order
+ * and rounded once.  Without items group_off and quarter_groups are read as
+ * by rspi_screen_loglike_sets.  A bulk copy that does not complete within 1 s
+ * sets *err = RSPI_ERR_TIMEOUT and the kernel returns.  Requires every
+ * entry's column <= part_w + 7 (check with rspi_sets_entries_check). */
 long long rspi_sets_part_sums_floats(long long n_sets, int n_ctas);
 /* *bad += the entries of entries[0, n) that are not a staged column
- * (< part_w + 8): the check of rspi_sets_fill's output before the first
- * launch. */
+ * (< part_w + 8): the check of the fill's output before the first
+ * launch; _check32: of the columns of counted entries. */
 int rspi_sets_entries_check(const unsigned short *entries, long long n, int part_w, int *bad,
                             cudaStream_t stream);
+int rspi_sets_entries_check32(const unsigned short *entries, long long n, int part_w, int *bad,
+                              cudaStream_t stream);
+int rspi_screen_loglike_items(const float *lslices_sets, long long num_rot, const double *init,
+                              const double *scales, const unsigned short *entries, int counted,
+                              const long long *group_off, const int *quarter_groups,
+                              const int *items, const int *item_off, float *seg_sums,
+                              int seg_slots, int seg_ctas, const int *set_frames,
+                              long long n_sets, int n_parts, int part_w, long long row_begin,
+                              long long row_end, float *ll, long long ll_stride,
+                              float *part_sums, int part_sums_ctas,
+                              unsigned long long *frame_max, int warps_per_cta, int n_ctas,
+                              int *err, cudaStream_t stream);
 int rspi_screen_loglike_sets(const float *lslices_sets, long long num_rot, const double *init,
                              const double *scales, const unsigned short *entries,
                              const long long *group_off, const int *quarter_groups,

@@ -29,8 +29,20 @@
 // is decomposed into permutations (Birkhoff-von Neumann; each permutation is
 // a perfect matching of the matrix's support, found by augmenting paths).
 // By Koenig's theorem the step count max(largest frame, largest class total)
-// is the fewest possible.  Entries: 16-bit local columns, four steps of a
+// is the fewest possible.  Entries: 16 bits, the local column (14 bits) and
+// the logarithm of a count of 1, 2, 4 or 8 photons (2 bits), four steps of a
 // lane per 8-byte group, groups of a (set, part) in one range (part-major).
+// A pixel of k photons takes an entry per binary digit of k (per 8 above), so
+// its value is gathered once or twice instead of k times: a sixth fewer slots
+// for frames of 50 to 50,000 photons, a twelfth for 2,000 (the gathers bound
+// the kernel; 39.1 to 38.1 ms for 72,900 states x 20,000 frames of 173
+// likelihood photons, 11.5 to 7.45 ms for 40,500 x 4,001 of 245, where the
+// heaviest set, a single warp's work, sets a tile's time and its pixels repeat
+// the most).  Where pixels seldom repeat, every entry is one photon and the
+// kernel has no multiplications (COUNTED = false).
+// A set far longer than a warp's share of a tile is cut into pieces taken by
+// several warps (ITEMS): 7.45 to 6.68 ms in the same case, 0.27 to 0.23 ms for
+// 7,056 states x 700 frames.
 #include "rspi_common.cuh"
 
 namespace {
@@ -49,11 +61,38 @@ __device__ __forceinline__ unsigned entry16_at(const unsigned short *__restrict_
 // ---------------------------------------------------------------------------
 // entry construction (once per dataset and geometry)
 // ---------------------------------------------------------------------------
+constexpr int COL_BITS = 14;         // local column of a set entry
+constexpr int MAX_LOG = 3;           // entries hold 2^0 .. 2^3 photons
 
-// counts[d * 32 + h * 8 + c]: frame d's photons in part h of local class c.
+// The frame's photons as (column, count): from the 16-bit lists, every copy
+// an entry of its own (COUNTED = false), or from the packed 32-bit entries
+// (column << 16 | count).
+template <bool COUNTED>
+struct Source {
+    const void *ent;
+    unsigned p_zero;     // columns from here on are padding
+    // count 0: no photon
+    __device__ __forceinline__ void at(long long rr, int lane, unsigned &c, unsigned &cnt) const {
+        if (COUNTED) {
+            const unsigned e = static_cast<const unsigned *>(ent)[rr * 32 + lane];
+            c = e >> 16;
+            cnt = c < p_zero ? e & 0xffffu : 0u;
+        } else {
+            c = entry16_at(static_cast<const unsigned short *>(ent), rr, lane);
+            cnt = c < p_zero ? 1u : 0u;
+        }
+    }
+    // slots of k photons: 8 at a time, then the binary digits
+    __device__ __forceinline__ static int slots(unsigned k) {
+        return (int)(k >> MAX_LOG) + __popc(k & ((1u << MAX_LOG) - 1u));
+    }
+};
+
+// counts[d * 32 + h * 8 + c]: frame d's entries in part h of local class c.
+template <bool COUNTED>
 __global__ void __launch_bounds__(BUILD_WARPS * 32)
-k_sets_counts(const unsigned short *__restrict__ ent16, const long long *__restrict__ row_off16,
-              long long n, int p_zero, int n_parts, int part_w, int *__restrict__ counts) {
+k_sets_counts(Source<COUNTED> src, const long long *__restrict__ row_off, long long n,
+              int n_parts, int part_w, int *__restrict__ counts) {
     __shared__ int cnt[BUILD_WARPS][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -61,18 +100,15 @@ k_sets_counts(const unsigned short *__restrict__ ent16, const long long *__restr
     for (long long d = warp; d < n; d += nwarp) {
         cnt[w][lane] = 0;
         __syncwarp();
-        const long long r0 = row_off16[d], nr = row_off16[d + 1] - r0;
-        for (long long r = 0; r < nr; ++r) {
-            const unsigned e = entry16_at(ent16, r0 + r, lane);
-            int key = 32;
-            if (e < (unsigned)p_zero) {
-                const int h = (int)(e / (unsigned)part_w);
-                key = h * 8 + (int)((e - (unsigned)(h * part_w)) & 7u);
+        for (long long r = row_off[d]; r < row_off[d + 1]; ++r) {
+            unsigned c, k;
+            src.at(r, lane, c, k);
+            if (k) {
+                const unsigned h = c / (unsigned)part_w;
+                atomicAdd(&cnt[w][h * 8 + ((c - h * part_w) & 7u)], src.slots(k));
             }
-            const unsigned m = __match_any_sync(RSPI_FULL_MASK, key);
-            if (key < 32 && lane == __ffs(m) - 1) cnt[w][key] += __popc(m);
-            __syncwarp();
         }
+        __syncwarp();
         counts[d * 32 + lane] = lane < n_parts * 8 ? cnt[w][lane] : 0;
         __syncwarp();
     }
@@ -361,14 +397,15 @@ __device__ bool perfect_matching(const int (&m)[8][8], int (&col_of)[8]) {
 // (the larger of its fullest frame and its fullest class), into
 // permutations (shared memory: packed classes of the eight lanes, 3 bits
 // each in 4-bit fields, the multiplicity and the first step of each); then
-// every lane places its frame's photons of the part, the k-th photon of
+// every lane places its frame's entries of the part, the k-th entry of
 // class c at the k-th step in which the lane reads class c, the zero column
 // part_w + c at that class's remaining steps below D_p, and from D_p on
 // (steps the kernel skips after group ceil(D_p / 4) of the quarter warp)
 // the zero column of its own class f.
+template <bool COUNTED>
 __global__ void __launch_bounds__(BUILD_WARPS * 32)
-k_sets_fill(const unsigned short *__restrict__ ent16, const long long *__restrict__ row_off16,
-            int p_zero, int n_parts, int part_w, const int *__restrict__ counts,
+k_sets_fill(Source<COUNTED> src, const long long *__restrict__ row_off, int n_parts, int part_w,
+            const int *__restrict__ counts,
             const int *__restrict__ set_frames, long long n_sets,
             const long long *__restrict__ goff, unsigned short *__restrict__ out,
             int *__restrict__ err) {
@@ -464,18 +501,22 @@ k_sets_fill(const unsigned short *__restrict__ ent16, const long long *__restric
             out[((g0 + step / 4) * 32 + lane) * 4 + (step & 3)] = (unsigned short)v;
         };
         if (d >= 0 && np > 0) {
-            const long long r0 = row_off16[d], r1 = row_off16[d + 1];
-            for (long long rr = r0; rr < r1; ++rr) {
+            for (long long rr = row_off[d]; rr < row_off[d + 1]; ++rr) {
                 for (int l2 = 0; l2 < 32; ++l2) {
-                    const unsigned e = entry16_at(ent16, rr, l2);
-                    if (e >= (unsigned)p_zero || (int)(e / (unsigned)part_w) != h) continue;
+                    unsigned e, k;
+                    src.at(rr, l2, e, k);
+                    if (k == 0 || (int)(e / (unsigned)part_w) != h) continue;
                     const unsigned loc = e - (unsigned)(h * part_w);
-                    const int st = next_step((int)(loc & 7u));
-                    if (st < 0) {
-                        rspi_flag(err, RSPI_ERR_CAPACITY);
-                        continue;
+                    while (k) {
+                        const int lg = min(31 - __clz((int)k), MAX_LOG);
+                        k -= 1u << lg;
+                        const int st = next_step((int)(loc & 7u));
+                        if (st < 0) {
+                            rspi_flag(err, RSPI_ERR_CAPACITY);
+                            break;
+                        }
+                        put(st, loc | (unsigned)lg << COL_BITS);
                     }
-                    put(st, loc);
                 }
             }
         }
@@ -555,14 +596,41 @@ __device__ __forceinline__ float4 f4_add(float4 a, float4 b) {
     return make_float4(lo.x, lo.y, hi.x, hi.y);
 }
 
-// The four photons of one group of a lane, summed as a tree of depth two:
-// (v0 + v1) + (v2 + v3), four rows each.
+// The four entries of one group of a lane, summed as a tree of depth two,
+// (v0 k0 + v1 k1) + (v2 k2 + v3 k3), four rows each.  The weight k is an
+// eighth of the entry's count, the two count bits under a fixed exponent
+// prefix (2^-3 .. 2^0): products with it are exact.
+constexpr float SUM_SCALE = 8.f;   // of the sums, at the end
+
+__device__ __forceinline__ float2 entry_weight(unsigned bits) {
+    const float k = __uint_as_float((bits & 0x1800000u) | 0x3e000000u);
+    return make_float2(k, k);
+}
+
+template <bool COUNTED>
 __device__ __forceinline__ float4 group_sum(const unsigned char *tile, uint2 e) {
-    const float4 v0 = *reinterpret_cast<const float4 *>(tile + ((e.x & 0xffffu) << 4));
-    const float4 v1 = *reinterpret_cast<const float4 *>(tile + ((e.x >> 16) << 4));
-    const float4 v2 = *reinterpret_cast<const float4 *>(tile + ((e.y & 0xffffu) << 4));
-    const float4 v3 = *reinterpret_cast<const float4 *>(tile + ((e.y >> 16) << 4));
-    return f4_add(f4_add(v0, v1), f4_add(v2, v3));
+    if (!COUNTED) {
+        const float4 v0 = *reinterpret_cast<const float4 *>(tile + ((e.x & 0xffffu) << 4));
+        const float4 v1 = *reinterpret_cast<const float4 *>(tile + ((e.x >> 16) << 4));
+        const float4 v2 = *reinterpret_cast<const float4 *>(tile + ((e.y & 0xffffu) << 4));
+        const float4 v3 = *reinterpret_cast<const float4 *>(tile + ((e.y >> 16) << 4));
+        return f4_add(f4_add(v0, v1), f4_add(v2, v3));
+    }
+    constexpr unsigned MASK = ((1u << COL_BITS) - 1u) << 4;
+    const float4 v0 = *reinterpret_cast<const float4 *>(tile + ((e.x << 4) & MASK));
+    const float4 v1 = *reinterpret_cast<const float4 *>(tile + ((e.x >> 12) & MASK));
+    const float4 v2 = *reinterpret_cast<const float4 *>(tile + ((e.y << 4) & MASK));
+    const float4 v3 = *reinterpret_cast<const float4 *>(tile + ((e.y >> 12) & MASK));
+    const float2 k0 = entry_weight(e.x << 9), k1 = entry_weight(e.x >> 7);
+    const float2 k2 = entry_weight(e.y << 9), k3 = entry_weight(e.y >> 7);
+    auto pair = [](float2 a, float2 ka, float2 b, float2 kb) {
+        return __ffma2_rn(b, kb, __fmul2_rn(a, ka));
+    };
+    const float2 lo = __fadd2_rn(pair(make_float2(v0.x, v0.y), k0, make_float2(v1.x, v1.y), k1),
+                                 pair(make_float2(v2.x, v2.y), k2, make_float2(v3.x, v3.y), k3));
+    const float2 hi = __fadd2_rn(pair(make_float2(v0.z, v0.w), k0, make_float2(v1.z, v1.w), k1),
+                                 pair(make_float2(v2.z, v2.w), k2, make_float2(v3.z, v3.w), k3));
+    return make_float4(lo.x, lo.y, hi.x, hi.y);
 }
 
 // Tensor memory (TMEM, 128 lanes x 512 columns of 32 bits per SM) as the
@@ -571,6 +639,7 @@ __device__ __forceinline__ float4 group_sum(const unsigned char *tile, uint2 e) 
 // lane), for the first TMEM_SETS sets; later sets use the global scratch.
 constexpr int TMEM_COLS = 512;
 constexpr int TMEM_SETS = 4 * (TMEM_COLS / 4);
+constexpr int SPLIT_SETS = 64;   // sets that may be cut into pieces (the first)
 
 __device__ __forceinline__ void tmem_fence_before() {
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -609,12 +678,14 @@ __device__ __forceinline__ float4 tmem_load4(unsigned taddr) {
 // its lane quarter in every part.  The last part adds the parts in FP64
 // before the final rounding, stores the four rows' likelihoods in column
 // 32 s + l and folds them into the column's argmax key (frame_max).
-template <int THREADS>
+template <int THREADS, bool COUNTED, bool ITEMS>
 __global__ void __launch_bounds__(THREADS, 1)
 k_screen_sets(const float4 *__restrict__ lsl4, int num_rot, const double *__restrict__ init,
               const double *__restrict__ scales, const uint2 *__restrict__ groups,
               const long long *__restrict__ goff, const int *__restrict__ qgroups,
-              const int *__restrict__ set_frames, int n_sets, int n_parts, int part_w,
+              const int4 *__restrict__ items, const int *__restrict__ item_off,
+              float4 *seg_sums, int seg_slots, const int *__restrict__ set_frames, int n_sets,
+              int n_parts, int part_w,
               long long row_begin, long long row_end, float *__restrict__ ll,
               long long ll_stride, float4 *part_sums, unsigned long long *__restrict__ frame_max,
               int *err) {
@@ -623,12 +694,15 @@ k_screen_sets(const float4 *__restrict__ lsl4, int num_rot, const double *__rest
     __shared__ int next_set[4];
     __shared__ int abort_flag;
     __shared__ unsigned tmem_slot;
+    __shared__ int seg_done[ITEMS ? SPLIT_SETS : 1];
     float4 *tile = reinterpret_cast<float4 *>(smem_raw);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned bytes = (unsigned)part_w * 16u;
     const unsigned mbar_a = smem_u32(&mbar), tile_a = smem_u32(tile);
     const unsigned long long keep = policy_evict_last(), stream_out = policy_evict_first();
     const bool split = n_parts > 1;   // running part sums (TMEM + scratch)
+    if (ITEMS)
+        for (int i = threadIdx.x; i < SPLIT_SETS; i += blockDim.x) seg_done[i] = 0;
     if (threadIdx.x < 8) tile[part_w + threadIdx.x] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (threadIdx.x == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar_a) : "memory");
@@ -726,17 +800,33 @@ k_screen_sets(const float4 *__restrict__ lsl4, int num_rot, const double *__rest
                     if (k < nt) ini[k] = init[(first + k) / num_rot];
             }
             while (true) {
-                int s = 0;
-                if (lane == 0) s = queue + n_queues * atomicAdd(&next_set[queue], 1);
-                s = __shfl_sync(RSPI_FULL_MASK, s, 0);
-                if (s >= n_sets) break;
-                const long long gi = (long long)h * n_sets + s;
-                const long long g0 = goff[gi], g1 = goff[gi + 1];
-                // the set runs ng groups; this lane's quarter warp stops after
-                // its own nq (<= ng): its later gathers are not issued, so
-                // they take no shared-memory wavefront
-                const int ng = (int)(g1 - g0);
-                const int nq = qgroups ? qgroups[gi * 4 + (lane >> 3)] : ng;
+                // set s from group g0 on: the warp runs ng groups; this lane's
+                // quarter warp stops after its own nq (<= ng): its later
+                // gathers are not issued, so they take no shared-memory
+                // wavefront
+                int s = 0, ng, nq;
+                long long g0;
+                unsigned piece = 0;
+                if (ITEMS) {
+                    if (lane == 0) s = atomicAdd(&next_set[queue], 1);
+                    s = __shfl_sync(RSPI_FULL_MASK, s, 0) + item_off[h * n_queues + queue];
+                    if (s >= item_off[h * n_queues + queue + 1]) break;
+                    const int4 *it = items + 2 * (long long)s;
+                    nq = reinterpret_cast<const int *>(it + 1)[lane >> 3];
+                    const int4 head = *it;
+                    s = head.x;
+                    g0 = head.y;
+                    ng = head.z;
+                    piece = (unsigned)head.w;
+                } else {
+                    if (lane == 0) s = queue + n_queues * atomicAdd(&next_set[queue], 1);
+                    s = __shfl_sync(RSPI_FULL_MASK, s, 0);
+                    if (s >= n_sets) break;
+                    const long long gi = (long long)h * n_sets + s;
+                    g0 = goff[gi];
+                    ng = (int)(goff[gi + 1] - g0);
+                    nq = qgroups ? qgroups[gi * 4 + (lane >> 3)] : ng;
+                }
                 float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), a1 = a0;
                 const uint2 *gp = groups + g0 * 32 + lane;
                 int k = 0;
@@ -745,13 +835,40 @@ k_screen_sets(const float4 *__restrict__ lsl4, int num_rot, const double *__rest
                 for (; k + 1 < ng; k += 2, gp += 64) {
                     const uint2 n0 = k + 2 < nq ? ld_entries(gp + 64, keep) : make_uint2(0, 0);
                     const uint2 n1 = k + 3 < nq ? ld_entries(gp + 96, keep) : make_uint2(0, 0);
-                    if (k < nq) a0 = f4_add(a0, group_sum(smem_raw, c0));
-                    if (k + 1 < nq) a1 = f4_add(a1, group_sum(smem_raw, c1));
+                    if (k < nq) a0 = f4_add(a0, group_sum<COUNTED>(smem_raw, c0));
+                    if (k + 1 < nq) a1 = f4_add(a1, group_sum<COUNTED>(smem_raw, c1));
                     c0 = n0;
                     c1 = n1;
                 }
-                if (k < nq) a0 = f4_add(a0, group_sum(smem_raw, c0));
-                const float4 sum = f4_add(a0, a1);
+                if (k < nq) a0 = f4_add(a0, group_sum<COUNTED>(smem_raw, c0));
+                float4 sum = f4_add(a0, a1);
+                if (ITEMS && piece >> 24 > 1u) {
+                    // a piece of a long set: the warp that finishes the last
+                    // piece adds them in FP64, in their order
+                    const int n_seg = (int)(piece >> 24);
+                    float4 *sp = seg_sums +
+                                 ((long long)blockIdx.x * seg_slots + (piece & 0xffffu)) * 32 +
+                                 lane;
+                    sp[(int)(piece >> 16 & 0xffu) * 32] = sum;
+                    __threadfence_block();
+                    __syncwarp();
+                    int done = 0;
+                    if (lane == 0) done = atomicAdd(&seg_done[s], 1);
+                    done = __shfl_sync(RSPI_FULL_MASK, done, 0);
+                    if (done != n_seg - 1) continue;
+                    __syncwarp();
+                    __threadfence_block();
+                    if (lane == 0) seg_done[s] = 0;   // for the next part
+                    double t[4] = {0., 0., 0., 0.};
+                    for (int q = 0; q < n_seg; ++q) {
+                        const float4 v = __ldcg(sp + q * 32);
+                        t[0] += (double)v.x;
+                        t[1] += (double)v.y;
+                        t[2] += (double)v.z;
+                        t[3] += (double)v.w;
+                    }
+                    sum = make_float4((float)t[0], (float)t[1], (float)t[2], (float)t[3]);
+                }
                 const int col = s * 32 + lane;
                 // this set's running sum: TMEM columns 4 (s / 4) of the lane
                 // quarter, or the scratch
@@ -784,7 +901,9 @@ k_screen_sets(const float4 *__restrict__ lsl4, int num_rot, const double *__rest
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     if (k < nt) {
-                        const float v = (float)(ini[k] * sc + ((double)pr[k] + (double)sm[k]));
+                        const double total = (double)pr[k] + (double)sm[k];
+                        const float v =
+                            (float)(ini[k] * sc + (COUNTED ? (double)SUM_SCALE * total : total));
                         st_f32_hint(ll + (first + k - row_begin) * ll_stride + col, v, stream_out);
                         const unsigned long long kk = argmax_key(v, (unsigned)(first + k));
                         key = kk > key ? kk : key;
@@ -804,13 +923,13 @@ k_screen_sets(const float4 *__restrict__ lsl4, int num_rot, const double *__rest
                      : "memory");
 }
 
-// bad += entries that are not a staged column (< part_w + 8).
+// bad += entries whose column is not a staged one (< part_w + 8).
 __global__ void k_sets_check(const unsigned short *__restrict__ e, long long n, int part_w,
-                             int *__restrict__ bad) {
+                             unsigned mask, int *__restrict__ bad) {
     const long long stride = (long long)gridDim.x * blockDim.x;
     int cnt = 0;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
-        cnt += (unsigned)e[i] >= (unsigned)(part_w + 8);
+        cnt += (e[i] & mask) >= (unsigned)(part_w + 8);
     cnt = warp_sum(cnt);
     if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(bad, cnt);
 }
@@ -842,16 +961,36 @@ __global__ void k_frame_max_finalize(unsigned long long *__restrict__ frame_max,
 
 }  // namespace
 
+static bool sets_columns_ok(int p_zero, int n_parts, int part_w, int part_w_max) {
+    return p_zero >= 0 && p_zero % 32 == 0 && p_zero + 32 <= 65536 && n_parts >= 1 &&
+           n_parts <= SETS_MAX_PARTS && part_w >= 8 && part_w % 8 == 0 &&
+           part_w <= part_w_max && (long long)n_parts * part_w >= p_zero;
+}
+
+template <bool COUNTED>
+static int sets_counts(const void *ent, const long long *row_off, long long n_data, int p_zero,
+                       int n_parts, int part_w, int *counts, cudaStream_t stream) {
+    if (!ent || !row_off || !counts || n_data <= 0 ||
+        !sets_columns_ok(p_zero, n_parts, part_w, COUNTED ? (1 << COL_BITS) - 8 : 0x7fffffff))
+        return RSPI_ERR_ARG;
+    k_sets_counts<COUNTED>
+        <<<rspi_blocks(n_data * 32, BUILD_WARPS * 32), BUILD_WARPS * 32, 0, stream>>>(
+            Source<COUNTED>{ent, (unsigned)p_zero}, row_off, n_data, n_parts, part_w, counts);
+    RSPI_RETURN_LAUNCH();
+}
+
 extern "C" int rspi_sets_counts(const unsigned short *entries16, const long long *row_off16,
                                 long long n_data, int p_zero, int n_parts, int part_w,
                                 int *counts, cudaStream_t stream) {
-    if (!entries16 || !row_off16 || !counts || n_data <= 0 || p_zero < 0 || p_zero % 32 ||
-        p_zero + 32 > 65536 || n_parts < 1 || n_parts > SETS_MAX_PARTS || part_w < 8 ||
-        part_w % 8 || (long long)n_parts * part_w < p_zero)
-        return RSPI_ERR_ARG;
-    k_sets_counts<<<rspi_blocks(n_data * 32, BUILD_WARPS * 32), BUILD_WARPS * 32, 0, stream>>>(
-        entries16, row_off16, n_data, p_zero, n_parts, part_w, counts);
-    RSPI_RETURN_LAUNCH();
+    return sets_counts<false>(entries16, row_off16, n_data, p_zero, n_parts, part_w, counts,
+                              stream);
+}
+
+extern "C" int rspi_sets_counts32(const unsigned int *entries32, const long long *row_off32,
+                                  long long n_data, int p_zero, int n_parts, int part_w,
+                                  int *counts, cudaStream_t stream) {
+    return sets_counts<true>(entries32, row_off32, n_data, p_zero, n_parts, part_w, counts,
+                             stream);
 }
 
 extern "C" int rspi_sets_group(const int *counts, const int *order, long long n, int n_parts,
@@ -876,27 +1015,55 @@ extern "C" int rspi_sets_steps(const int *counts, const int *set_frames, long lo
     RSPI_RETURN_LAUNCH();
 }
 
+template <bool COUNTED>
+static int sets_fill(const void *ent, const long long *row_off, int p_zero, int n_parts,
+                     int part_w, const int *counts, const int *set_frames, long long n_sets,
+                     const long long *group_off, unsigned short *entries, int *err,
+                     cudaStream_t stream) {
+    if (!ent || !row_off || !counts || !set_frames || !group_off || !entries || n_sets <= 0 ||
+        n_sets > 0x3ffffffLL ||
+        !sets_columns_ok(p_zero, n_parts, part_w, COUNTED ? (1 << COL_BITS) - 8 : 0xffff - 8) ||
+        (reinterpret_cast<uintptr_t>(entries) & 7) != 0)
+        return RSPI_ERR_ARG;
+    k_sets_fill<COUNTED><<<rspi_blocks(n_sets * n_parts * 32, BUILD_WARPS * 32),
+                           BUILD_WARPS * 32, 0, stream>>>(
+        Source<COUNTED>{ent, (unsigned)p_zero}, row_off, n_parts, part_w, counts, set_frames,
+        n_sets, group_off, entries, err);
+    RSPI_RETURN_LAUNCH();
+}
+
 extern "C" int rspi_sets_fill(const unsigned short *entries16, const long long *row_off16,
                               int p_zero, int n_parts, int part_w, const int *counts,
                               const int *set_frames, long long n_sets, const long long *group_off,
                               unsigned short *entries, int *err, cudaStream_t stream) {
-    if (!entries16 || !row_off16 || !counts || !set_frames || !group_off || !entries ||
-        n_sets <= 0 || n_sets > 0x3ffffffLL || p_zero < 0 || p_zero % 32 ||
-        p_zero + 32 > 65536 || n_parts < 1 || n_parts > SETS_MAX_PARTS || part_w < 8 ||
-        part_w % 8 || part_w + 8 > 0xffff || (long long)n_parts * part_w < p_zero ||
-        (reinterpret_cast<uintptr_t>(entries) & 7) != 0)
-        return RSPI_ERR_ARG;
-    k_sets_fill<<<rspi_blocks(n_sets * n_parts * 32, BUILD_WARPS * 32), BUILD_WARPS * 32, 0,
-                  stream>>>(entries16, row_off16, p_zero, n_parts, part_w, counts, set_frames,
-                            n_sets, group_off, entries, err);
+    return sets_fill<false>(entries16, row_off16, p_zero, n_parts, part_w, counts, set_frames,
+                            n_sets, group_off, entries, err, stream);
+}
+
+extern "C" int rspi_sets_fill32(const unsigned int *entries32, const long long *row_off32,
+                                int p_zero, int n_parts, int part_w, const int *counts,
+                                const int *set_frames, long long n_sets,
+                                const long long *group_off, unsigned short *entries, int *err,
+                                cudaStream_t stream) {
+    return sets_fill<true>(entries32, row_off32, p_zero, n_parts, part_w, counts, set_frames,
+                           n_sets, group_off, entries, err, stream);
+}
+
+static int sets_check(const unsigned short *entries, long long n, int part_w, int part_w_max,
+                      unsigned mask, int *bad, cudaStream_t stream) {
+    if (!entries || !bad || n <= 0 || part_w < 8 || part_w > part_w_max) return RSPI_ERR_ARG;
+    k_sets_check<<<rspi_blocks(n, 256), 256, 0, stream>>>(entries, n, part_w, mask, bad);
     RSPI_RETURN_LAUNCH();
 }
 
 extern "C" int rspi_sets_entries_check(const unsigned short *entries, long long n, int part_w,
                                        int *bad, cudaStream_t stream) {
-    if (!entries || !bad || n <= 0 || part_w < 8 || part_w + 8 > 0xffff) return RSPI_ERR_ARG;
-    k_sets_check<<<rspi_blocks(n, 256), 256, 0, stream>>>(entries, n, part_w, bad);
-    RSPI_RETURN_LAUNCH();
+    return sets_check(entries, n, part_w, 0xffff - 8, 0xffffu, bad, stream);
+}
+
+extern "C" int rspi_sets_entries_check32(const unsigned short *entries, long long n, int part_w,
+                                         int *bad, cudaStream_t stream) {
+    return sets_check(entries, n, part_w, (1 << COL_BITS) - 8, (1u << COL_BITS) - 1u, bad, stream);
 }
 
 extern "C" long long rspi_sets_part_sums_floats(long long n_sets, int n_ctas) {
@@ -906,17 +1073,34 @@ extern "C" long long rspi_sets_part_sums_floats(long long n_sets, int n_ctas) {
     return (long long)n_ctas * extra * 32 * 4;
 }
 
-extern "C" int rspi_screen_loglike_sets(const float *lslices_sets, long long num_rot,
-                                        const double *init, const double *scales,
-                                        const unsigned short *entries, const long long *group_off,
-                                        const int *quarter_groups, const int *set_frames,
-                                        long long n_sets, int n_parts,
-                                        int part_w, long long row_begin, long long row_end,
-                                        float *ll, long long ll_stride, float *part_sums,
-                                        int part_sums_ctas, unsigned long long *frame_max,
-                                        int warps_per_cta, int n_ctas, int *err,
-                                        cudaStream_t stream) {
-    if (!lslices_sets || !init || !scales || !entries || !group_off || !set_frames || !ll ||
+template <int THREADS, bool COUNTED, bool ITEMS>
+static int screen_sets(int n_ctas, int warps, size_t smem, cudaStream_t stream, const float4 *src,
+                       int num_rot, const double *init, const double *scales, const uint2 *ent,
+                       const long long *goff, const int *qg, const int4 *items,
+                       const int *item_off, float4 *seg_sums, int seg_slots,
+                       const int *set_frames, int n_sets, int n_parts, int part_w,
+                       long long row_begin, long long row_end, float *ll, long long ll_stride,
+                       float4 *ps, unsigned long long *frame_max, int *err) {
+    static RspiSmemOptIn optin;
+    if (!rspi_smem_optin((const void *)k_screen_sets<THREADS, COUNTED, ITEMS>, smem, optin))
+        return RSPI_ERR_CUDA;
+    k_screen_sets<THREADS, COUNTED, ITEMS><<<n_ctas, warps * 32, smem, stream>>>(
+        src, num_rot, init, scales, ent, goff, qg, items, item_off, seg_sums, seg_slots,
+        set_frames, n_sets, n_parts, part_w, row_begin, row_end, ll, ll_stride, ps, frame_max,
+        err);
+    RSPI_RETURN_LAUNCH();
+}
+
+static int screen_sets_any(const float *lslices_sets, long long num_rot, const double *init,
+                           const double *scales, const unsigned short *entries, bool counted,
+                           const long long *group_off, const int *quarter_groups,
+                           const int *items, const int *item_off, float *seg_sums,
+                           int seg_slots, int seg_ctas, const int *set_frames,
+                           long long n_sets, int n_parts, int part_w, long long row_begin,
+                           long long row_end, float *ll, long long ll_stride, float *part_sums,
+                           int part_sums_ctas, unsigned long long *frame_max, int warps_per_cta,
+                           int n_ctas, int *err, cudaStream_t stream) {
+    if (!lslices_sets || !init || !scales || !entries || !set_frames || !ll ||
         !frame_max || !err || n_sets <= 0 || n_sets > 0x3ffffffLL || num_rot <= 0 ||
         num_rot > 0x7fffffffLL || row_begin < 0 || row_end < row_begin ||
         row_end > 0x7fffffffLL || n_parts < 1 || n_parts > SETS_MAX_PARTS || part_w < 8 ||
@@ -941,21 +1125,53 @@ extern "C" int rspi_screen_loglike_sets(const float *lslices_sets, long long num
     float4 *ps = n_parts > 1 ? reinterpret_cast<float4 *>(part_sums) : nullptr;
     const float4 *src = reinterpret_cast<const float4 *>(lslices_sets);
     const uint2 *ent = reinterpret_cast<const uint2 *>(entries);
-    if (warps_per_cta <= 16) {
-        static RspiSmemOptIn optin;
-        if (!rspi_smem_optin((const void *)k_screen_sets<512>, smem, optin)) return RSPI_ERR_CUDA;
-        k_screen_sets<512><<<n_ctas, warps_per_cta * 32, smem, stream>>>(
-            src, (int)num_rot, init, scales, ent, group_off, quarter_groups, set_frames,
-            (int)n_sets, n_parts, part_w, row_begin, row_end, ll, ll_stride, ps, frame_max, err);
-    } else {
-        static RspiSmemOptIn optin;
-        if (!rspi_smem_optin((const void *)k_screen_sets<1024>, smem, optin))
-            return RSPI_ERR_CUDA;
-        k_screen_sets<1024><<<n_ctas, warps_per_cta * 32, smem, stream>>>(
-            src, (int)num_rot, init, scales, ent, group_off, quarter_groups, set_frames,
-            (int)n_sets, n_parts, part_w, row_begin, row_end, ll, ll_stride, ps, frame_max, err);
-    }
-    RSPI_RETURN_LAUNCH();
+    if (items && seg_slots > 0 && n_ctas > seg_ctas) n_ctas = seg_ctas;
+    const auto run =
+        warps_per_cta <= 16
+            ? (items ? (counted ? screen_sets<512, true, true> : screen_sets<512, false, true>)
+                     : (counted ? screen_sets<512, true, false> : screen_sets<512, false, false>))
+            : (items ? (counted ? screen_sets<1024, true, true> : screen_sets<1024, false, true>)
+                     : (counted ? screen_sets<1024, true, false> : screen_sets<1024, false, false>));
+    return run(n_ctas, warps_per_cta, smem, stream, src, (int)num_rot, init, scales, ent,
+               group_off, quarter_groups, reinterpret_cast<const int4 *>(items), item_off,
+               reinterpret_cast<float4 *>(seg_sums), seg_slots, set_frames, (int)n_sets, n_parts,
+               part_w, row_begin, row_end, ll, ll_stride, ps, frame_max, err);
+}
+
+extern "C" int rspi_screen_loglike_sets(const float *lslices_sets, long long num_rot,
+                                        const double *init, const double *scales,
+                                        const unsigned short *entries, const long long *group_off,
+                                        const int *quarter_groups, const int *set_frames,
+                                        long long n_sets, int n_parts,
+                                        int part_w, long long row_begin, long long row_end,
+                                        float *ll, long long ll_stride, float *part_sums,
+                                        int part_sums_ctas, unsigned long long *frame_max,
+                                        int warps_per_cta, int n_ctas, int *err,
+                                        cudaStream_t stream) {
+    if (!group_off) return RSPI_ERR_ARG;
+    return screen_sets_any(lslices_sets, num_rot, init, scales, entries, false, group_off,
+                           quarter_groups, nullptr, nullptr, nullptr, 0, 0, set_frames, n_sets,
+                           n_parts, part_w, row_begin, row_end, ll, ll_stride, part_sums,
+                           part_sums_ctas, frame_max, warps_per_cta, n_ctas, err, stream);
+}
+
+extern "C" int rspi_screen_loglike_items(
+    const float *lslices_sets, long long num_rot, const double *init, const double *scales,
+    const unsigned short *entries, int counted, const long long *group_off,
+    const int *quarter_groups, const int *items, const int *item_off,
+    float *seg_sums, int seg_slots, int seg_ctas, const int *set_frames, long long n_sets,
+    int n_parts, int part_w, long long row_begin, long long row_end, float *ll,
+    long long ll_stride, float *part_sums, int part_sums_ctas, unsigned long long *frame_max,
+    int warps_per_cta, int n_ctas, int *err, cudaStream_t stream) {
+    if ((!items && !group_off) || (items && !item_off) || seg_slots < 0 || seg_slots > 0xffff ||
+        (seg_slots > 0 && (!seg_sums || seg_ctas < 1)) ||
+        (reinterpret_cast<uintptr_t>(items) & 15) != 0 ||
+        (reinterpret_cast<uintptr_t>(seg_sums) & 15) != 0)
+        return RSPI_ERR_ARG;
+    return screen_sets_any(lslices_sets, num_rot, init, scales, entries, counted != 0, group_off,
+                           quarter_groups, items, item_off, seg_sums, seg_slots, seg_ctas, set_frames,
+                           n_sets, n_parts, part_w, row_begin, row_end, ll, ll_stride, part_sums,
+                           part_sums_ctas, frame_max, warps_per_cta, n_ctas, err, stream);
 }
 
 extern "C" int rspi_frame_max_finalize(unsigned long long *frame_max, const int *frame_of_col,

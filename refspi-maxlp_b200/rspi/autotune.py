@@ -35,7 +35,10 @@ WARPS_FOUR_ROW = (16, 24, 32)
 def key(es):
     name = torch.cuda.get_device_name(es.device)
     ent = es.ll if es.form == 'fp64' else es.ll16
-    return '%s|%s|%s|%d|%d|%d|%d' % (name, es.form, es.kernel, es.p_row, es.n_rows,
+    wide = es.wide or {}
+    kernel = es.kernel + ('-counted' if wide.get('counted') else '') + \
+        ('-cut' if wide.get('seg_slots') else '')
+    return '%s|%s|%s|%d|%d|%d|%d' % (name, es.form, kernel, es.p_row, es.n_rows,
                                      es.ph.num_data, ent['total_rows'])
 
 

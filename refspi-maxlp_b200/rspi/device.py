@@ -28,6 +28,19 @@ QUAD4_SMEM = 227 * 1024 - 1024   # shared bytes of the four-row tile (kernel lim
 QUAD4_MAX_PARTS = 4              # column parts of the four-row tile
 QUAD4_COLS = (QUAD4_SMEM // 16 - 8) // 8 * 8   # most columns of one part
 SETS_SWEEPS = 4                  # pair sweeps of the frame grouping (rspi_sets_group)
+SETS_COUNTED_COLS = (1 << 14) - 8   # most columns of a part with counted entries
+# Entries of several photons are taken where they leave out one entry in 14
+# or more, since each is multiplied by its count: 72,900 states x 8,000 frames
+# of 173 likelihood photons, 8.4% fewer entries, 15.9 ms for 16.3 (single
+# entries); of 104, 5.5% fewer, 11.1 for 11.0; of 52, 3% fewer, 7.2 for 7.0.
+COUNT_GAIN = 14
+SPLIT_SETS = 64                  # sets the frame-set kernel may cut (its limit)
+SPLIT_WARPS = 32                 # warps sharing a tile (the widest CTA)
+# A set longer than three warps' shares of its part is cut into pieces of a
+# share.  Below that the other warps' sets fill the time, and the pieces'
+# larger headers cost more: 1,000 frames, longest set 2.3 shares, 0.68 ms
+# whole and 0.70 cut; 4,001 frames, longest 9 shares, 7.45 whole and 6.68 cut.
+SPLIT_SHARES = 3
 PIXEL_MAP_MAX_ROT = 1024         # rotation tables the M-step's pixel map serves
 PIXEL_MAP_MAX = 1 << 26          # (rotation, detector pixel) entries of that map
 
@@ -256,6 +269,8 @@ class EStep:
                  slice_math=None, set_order='grouped'):
         if form not in ('fp64', 'screen', 'dense'):
             raise ValueError('form must be fp64, screen or dense')
+        # entries of several photons: only where the layout is left to choose
+        self.count_entries = kernel is None
         if kernel is None:   # default likelihood kernel of each form
             kernel = 'sets' if form == 'screen' else 'stream'
         kernels = {'fp64': ('stream', 'dynamic'), 'screen': ('stream', 'quad4', 'sets'),
@@ -552,21 +567,35 @@ class EStep:
 
     def _sets_entries(self):
         """Entries of the frame-set kernel: frames in decreasing order of
-        their likelihood-pixel photons, grouped per 256 ranks into quarter
+        their entries, grouped per 256 ranks into quarter
         warps whose class totals stay close to their mean and quarters of
         alike cost four to a set (``set_order='grouped'``), or lane 8 p + f
         of set s the frame of rank 32 s + p + 4 f (``'rank'``).  Per (set,
         column part) a step schedule
         in which a quarter warp's eight lanes read eight distinct bank
         classes (rspi_sets_steps / rspi_sets_fill); one FP32 running sum per
-        (CTA, column) between parts when there are several."""
-        l16, n, dev, s = self.ll16, self.ph.num_data, self.device, cur_stream()
+        (CTA, column) between parts when there are several.
+
+        An entry is a photon, or, when the kernel was not asked for by name
+        and that leaves out one entry in COUNT_GAIN or more, up to eight
+        photons of a pixel (rspi_sets_counts32)."""
+        ll, n, dev, s = self.ll, self.ph.num_data, self.device, cur_stream()
         pz = self.p_row - 32
         parts, part_w = self._quad4_parts()
         counts = torch.empty(n * 32, dtype=_i32, device=dev)
-        call('rspi_sets_counts', ptr(l16['entries']), ptr(l16['row_off']), n, pz, parts, part_w,
-             ptr(counts), s)
-        tot = self.ll['frame_sel_photons']
+        counted = self.count_entries and part_w <= SETS_COUNTED_COLS
+        if counted:
+            call('rspi_sets_counts32', ptr(ll['entries']), ptr(ll['row_off']), n, pz, parts,
+                 part_w, ptr(counts), s)
+            tot = counts.view(n, 32).sum(1)
+            phot = ll['frame_sel_photons'].sum()
+            counted = bool((COUNT_GAIN * (phot - tot.sum()) >= phot).item())
+        if not counted:
+            ll = self.ll16
+            call('rspi_sets_counts', ptr(ll['entries']), ptr(ll['row_off']), n, pz, parts, part_w,
+                 ptr(counts), s)
+            tot = self.ll['frame_sel_photons']
+        form = '32' if counted else ''
         order = torch.argsort(-tot, stable=True)
         n_sets = (n + 31) // 32
         k = torch.arange(n_sets * 32, device=dev, dtype=_i64)
@@ -592,12 +621,12 @@ class EStep:
         total = int(goff[-1].item())
         # every slot starts at the zero column part_w (class 0), a valid index
         entries = torch.full((max(1, total) * 128,), part_w, dtype=torch.int16, device=dev)
-        call('rspi_sets_fill', ptr(l16['entries']), ptr(l16['row_off']), pz, parts, part_w,
+        call('rspi_sets_fill' + form, ptr(ll['entries']), ptr(ll['row_off']), pz, parts, part_w,
              ptr(counts), ptr(set_frames), n_sets, ptr(goff), ptr(entries), ptr(self.ph.err.t),
              s)
         self.ph.err.check('frame-set entries')
         bad = torch.zeros(1, dtype=_i32, device=dev)
-        call('rspi_sets_entries_check', ptr(entries), max(1, total) * 128, part_w, ptr(bad), s)
+        call('rspi_sets_entries_check' + form, ptr(entries), max(1, total) * 128, part_w, ptr(bad), s)
         if int(bad.item()) != 0:
             raise RuntimeError('%d frame-set entries outside the staged part' % int(bad.item()))
         # each frame's FP32 summation length for the candidate threshold:
@@ -613,11 +642,53 @@ class EStep:
                 torch.cuda.get_device_properties(dev).multi_processor_count
             ps = torch.empty(self.lib.rspi_sets_part_sums_floats(n_sets, ps_ctas),
                              dtype=torch.float32, device=dev)
+        items, item_off, slots = self._sets_items(groups, qgroups, goff, parts, n_sets)
+        seg_ctas = self.n_ctas if self.n_ctas > 0 else \
+            torch.cuda.get_device_properties(dev).multi_processor_count
+        seg = torch.empty(seg_ctas * slots * 128, dtype=torch.float32, device=dev) \
+            if slots else None
         return dict(entries=entries, group_off=goff, quarter_groups=qgroups,
-                    total_groups=total, tile=4, sets=True,
+                    total_groups=total, tile=4, sets=True, counted=counted, items=items,
+                    item_off=item_off, seg_sums=seg, seg_slots=slots, seg_ctas=seg_ctas,
                     set_frames=set_frames, col_of_frame=col_of_frame, n_sets=n_sets,
                     frame_groups=frame_groups, n_parts=parts, part_w=part_w, part_sums=ps,
                     part_sums_ctas=ps_ctas, counts=counts)
+
+    @staticmethod
+    def _sets_items(groups, qgroups, goff, parts, n_sets):
+        """The frame-set kernel's work items (rspi_screen_loglike_items): a
+        set of a part, or, of the first SPLIT_SETS sets, an even piece of one
+        longer than SPLIT_SHARES warps' shares of the part's groups.  Returns
+        (items, item_off, seg_slots), (None, None, 0) when no set is cut."""
+        dev = groups.device
+        g = groups.view(parts, n_sets).to(_i64)
+        share = (g.sum(1, keepdim=True) // SPLIT_WARPS).clamp(min=1)
+        s = torch.arange(n_sets, device=dev)
+        n_seg = torch.where((s < SPLIT_SETS) & (g > SPLIT_SHARES * share),
+                            (g + share - 1) // share, 1).clamp(max=127)
+        queues = 4 if parts > 1 else 1
+        pos = torch.argsort(s % queues, stable=True)      # sets queue by queue
+        at = (torch.arange(parts, device=dev)[:, None] * n_sets + pos).view(-1)
+        g, n_seg = g.view(-1), n_seg.view(parts, n_sets)
+        split = torch.where(n_seg > 1, n_seg, 0)
+        base = (split.cumsum(1) - split).view(-1)
+        off = torch.zeros(parts * queues + 1, dtype=_i64, device=dev)
+        off[1:] = torch.stack([n_seg[:, q::queues].sum(1) for q in range(queues)],
+                              1).view(-1).cumsum(0)
+        n_seg = n_seg.view(-1)
+        n_items, slots = torch.stack([off[-1], split.sum(1).max()]).tolist()
+        if slots == 0:
+            return None, None, 0
+        rep = torch.repeat_interleave(at, n_seg[at], output_size=n_items)
+        first = n_seg[at].cumsum(0) - n_seg[at]
+        k = torch.arange(n_items, device=dev) - \
+            torch.repeat_interleave(first, n_seg[at], output_size=n_items)
+        k0, k1 = g[rep] * k // n_seg[rep], g[rep] * (k + 1) // n_seg[rep]
+        quarters = qgroups.view(-1, 4)[rep].to(_i64) - k0[:, None]
+        quarters = torch.minimum(quarters.clamp(min=0), (k1 - k0)[:, None])
+        items = torch.cat([torch.stack([rep % n_sets, goff[rep] + k0, k1 - k0,
+                                        base[rep] | k << 16 | n_seg[rep] << 24], 1), quarters], 1)
+        return items.to(_i32).contiguous(), off.to(_i32), slots
 
     def _eps_rows(self):
         """Prefix sums of each frame's FP32 summation length for the
@@ -748,12 +819,12 @@ class EStep:
                  self.n_ctas, cur_stream())
         elif self.kernel == 'sets':
             w = self.wide
-            if w['n_parts'] > 1 and self.n_ctas > 0 and self.n_ctas != w['part_sums_ctas']:
+            if self.n_ctas > 0 and self.n_ctas != w['seg_ctas']:
                 w = self.wide = self._sets_entries()
-            call('rspi_screen_loglike_sets', ptr(lsl), self.num_rot, ptr(self.init),
-                 ptr(self.ph.scales), ptr(w['entries']), ptr(w['group_off']),
-                 ptr(w['quarter_groups']), ptr(w['set_frames']), w['n_sets'], w['n_parts'],
-                 w['part_w'], r0, r1,
+            call('rspi_screen_loglike_items', ptr(lsl), self.num_rot, ptr(self.init),
+                 ptr(self.ph.scales), ptr(w['entries']), int(w['counted']), ptr(w['group_off']),
+                 ptr(w['quarter_groups']), ptr(w['items']), ptr(w['item_off']), ptr(w['seg_sums']), w['seg_slots'], w['seg_ctas'],
+                 ptr(w['set_frames']), w['n_sets'], w['n_parts'], w['part_w'], r0, r1,
                  ptr(self.prob[r0]), self.n_cols, ptr(w['part_sums']), w['part_sums_ctas'],
                  ptr(self.frame_max), self.warps, self.n_ctas, ptr(self.ph.err.t), cur_stream())
         elif self.kernel == 'stream' and self.form == 'screen':

@@ -41,6 +41,7 @@ SIGNATURES = {
     'rspi_maxlp_pixel_frames': (I, [I, L, P, L] + [P] * 7 + [L, P, P, P, P, P, P]),
     'rspi_maxlp_pixel_values': (I, [P, L, P, P, L, I, D, P, P, P]),
     'rspi_sets_entries_check': (I, [P, L, I, P, P]),
+    'rspi_sets_entries_check32': (I, [P, L, I, P, P]),
     'rspi_sim_views': (I, [P, P, I, L, L, P, P, P, P, D, D, D, I, P, P, P]),
     'rspi_sim_counts': (I, [P, L, L, P, P, I, ctypes.c_ulonglong, P, P, P, P]),
     'rspi_sim_poisson': (I, [P, L, ctypes.c_ulonglong, ctypes.c_ulonglong, P, P, P]),
@@ -75,12 +76,16 @@ SIGNATURES = {
     'rspi_phase_proj_real': (I, [P, P, P, P, L, P]),
     'rspi_phase_refine': (I, [P, P, P, P, P, L, I, I, P]),
     'rspi_sets_counts': (I, [P, P, L, I, I, I, P, P]),
+    'rspi_sets_counts32': (I, [P, P, L, I, I, I, P, P]),
     'rspi_sets_group': (I, [P, P, L, I, I, P, P, P]),
     'rspi_sets_steps': (I, [P, P, L, I, P, P, P]),
     'rspi_sets_fill': (I, [P, P, I, I, I, P, P, L, P, P, P, P]),
+    'rspi_sets_fill32': (I, [P, P, I, I, I, P, P, L, P, P, P, P]),
     'rspi_holo_quads32': (I, [P, L, L, P, P]),
     'rspi_rot_log_slices_sets': (I, [P, P, L, L, P, L, P, P, L, I, I, L, L, P, P, P]),
     'rspi_sets_part_sums_floats': (L, [L, I]),
+    'rspi_screen_loglike_items': (I, [P, L, P, P, P, I, P, P, P, P, P, I, I, P, L, I, I, L, L, P, L,
+                                      P, I, P, I, I, P, P]),
     'rspi_screen_loglike_sets': (I, [P, L, P, P, P, P, P, P, L, I, I, L, L, P, L, P, I, P, I,
                                      I, P, P]),
     'rspi_frame_max_finalize': (I, [P, P, L, P, P, P]),
@@ -151,7 +156,9 @@ KERNELS_PER_CALL = {
     'rspi_loglike_stream': 1, 'rspi_posterior_pairs': 3,
     'rspi_entries16_check': 1, 'rspi_emc_nll': 2, 'rspi_emc_nll_grid': 2, 'rspi_cdft2': 2, 'rspi_phase_support': 5,
     'rspi_phase_proj_fourier': 1, 'rspi_phase_proj_real': 3, 'rspi_sets_counts': 1, 'rspi_sets_group': 1, 'rspi_sets_steps': 1,
-    'rspi_sets_fill': 1, 'rspi_rot_log_slices_sets': 1, 'rspi_holo_quads32': 1, 'rspi_sets_part_sums_floats': 0,
+    'rspi_sets_fill': 1, 'rspi_sets_counts32': 1, 'rspi_sets_fill32': 1, 'rspi_sets_entries_check32': 1,
+    'rspi_screen_loglike_items': 1,
+    'rspi_rot_log_slices_sets': 1, 'rspi_holo_quads32': 1, 'rspi_sets_part_sums_floats': 0,
     'rspi_screen_loglike_sets': 1, 'rspi_frame_max_finalize': 1,
     'rspi_screen_candidates_cols': 4, 'rspi_rescore_cols': 5, 'rspi_nll': 2, 'rspi_nll_grid': 2, 'rspi_screen_candidates_noalloc': 3, 'rspi_merge_coverage': 1, 'rspi_merge': 2, 'rspi_merge_rows': 2,
     'rspi_dense_frames': 1, 'rspi_rot_log_split': 1, 'rspi_dense_loglike': 1,
