@@ -463,6 +463,53 @@ k_rescore_direct(const int *__restrict__ cand_d, const int *__restrict__ cand_r,
     }
 }
 
+// One FP64 rotated slice row: rot_log_value of the likelihood pixels (the
+// same operations), RR_COLS columns of a thread at a time so that their
+// loads are in flight together; 0 from n_sel on.  The row leaves L1 little
+// room beside it, so the corner loads' latency bounds the build (FP64 pipe
+// 25% busy).  4,500 rows of 24,928 pixels with 190 candidates each, of ~300
+// entry slots: 1.57 ms with a column and an entry at a time, 1.43 with two
+// columns, 1.40 with four entries in flight as well (three and four columns,
+// eight entries: 1.45 to 1.48, registers spill).
+constexpr int RR_COLS = 2;
+constexpr int RR_BATCH = 4;   // entries of a candidate in flight
+__device__ __forceinline__ void rot_log_row(const double *__restrict__ w, int size, float inv_size,
+                                            double ac, double as, const double *__restrict__ bg,
+                                            const int *__restrict__ sel_pix, int n_sel, int p_pad,
+                                            double *sl) {
+    const int cen = size / 2;
+    for (int c0 = threadIdx.x; c0 < p_pad; c0 += RR_COLS * blockDim.x) {
+        int at[RR_COLS];           // first corner; -1: outside the detector, -2: no column
+        double t[RR_COLS];
+#pragma unroll
+        for (int u = 0; u < RR_COLS; ++u) {
+            const int c = c0 + u * (int)blockDim.x;
+            const int p = c < n_sel ? sel_pix[c] : 0;
+            int x, y;
+            pixel_xy(p, size, inv_size, x, y);
+            const double xc = (double)(x - cen), yc = (double)(y - cen);
+            const double tx = xadd(xsub(xmul(xc, ac), xmul(yc, as)), (double)cen);
+            const double ty = xadd(xadd(xmul(xc, as), xmul(yc, ac)), (double)cen);
+            const double fxl = floor(tx), fyl = floor(ty);
+            const bool in = !(fxl < 0. || fxl > size - 2 || fyl < 0. || fyl > size - 2);
+            at[u] = c >= n_sel ? -2 : in ? (int)fxl * size + (int)fyl : -1;
+            const double fx = tx - fxl, fy = ty - fyl, cx = 1. - fx, cy = 1. - fy;
+            const double *r0 = w + max(at[u], 0);
+            double v = xmul(xmul(r0[0], cx), cy);
+            v = xadd(v, xmul(xmul(r0[size], fx), cy));
+            v = xadd(v, xmul(xmul(r0[1], cx), fy));
+            v = xadd(v, xmul(xmul(r0[size + 1], fx), fy));
+            t[u] = xadd(v, bg[p]);
+        }
+#pragma unroll
+        for (int u = 0; u < RR_COLS; ++u) {
+            const int c = c0 + u * (int)blockDim.x;
+            const double v = at[u] < 0 || t[u] < 1.e-20 ? -1000. : log(t[u]);
+            if (c < p_pad) sl[c] = at[u] == -2 ? 0. : v;
+        }
+    }
+}
+
 // One CTA per likelihood row with candidates: the row's FP64 rotated slice
 // is computed into shared memory with rot_log_value (as k_rot_log_js does),
 // then each warp rescores candidate frames exactly as the FP64 form sums
@@ -546,16 +593,7 @@ k_rescore_rows(const long long *__restrict__ row_off, const int *__restrict__ ro
             direct = s_work * nw < p_pad * min(b - a, (long long)nw);
         }
         if (!direct) {
-            for (long long c = threadIdx.x; c < p_pad; c += blockDim.x) {
-                double v = 0.;
-                if (c < n_sel) {
-                    const int p = sel_pix[c];
-                    int x, y;
-                    pixel_xy(p, size, inv_size, x, y);
-                    v = rot_log_value(w, x, y, size, ac, as, bg[p]);
-                }
-                sl[c] = v;
-            }
+            rot_log_row(w, size, inv_size, ac, as, bg, sel_pix, (int)n_sel, (int)p_pad, sl);
         }
         __syncthreads();
         // the likelihood-pixel value of entry column c (0 past n_sel, as
@@ -609,7 +647,18 @@ k_rescore_rows(const long long *__restrict__ row_off, const int *__restrict__ ro
                     const long long cq1 = __shfl_sync(RSPI_FULL_MASK, q1, c);
                     double acc = 0.;
                     const unsigned *ep = ent32 + cq0 * 32 + lane;
-                    for (long long q = cq0; q < cq1; ++q, ep += 32) {
+                    long long q = cq0;
+                    if (!direct) {   // RR_BATCH entries in flight, added in their order
+                        for (; q + RR_BATCH <= cq1; q += RR_BATCH, ep += 32 * RR_BATCH) {
+                            unsigned e[RR_BATCH];
+#pragma unroll
+                            for (int u = 0; u < RR_BATCH; ++u) e[u] = __ldg(ep + 32 * u);
+#pragma unroll
+                            for (int u = 0; u < RR_BATCH; ++u)
+                                acc = fma((double)(e[u] & 0xffffu), sl[min(e[u] >> 16, cmax)], acc);
+                        }
+                    }
+                    for (; q < cq1; ++q, ep += 32) {
                         const unsigned e = __ldg(ep);
                         acc = fma((double)(e & 0xffffu), value(e >> 16), acc);
                     }
