@@ -41,8 +41,8 @@
 // the most).  Where pixels seldom repeat, every entry is one photon and the
 // kernel has no multiplications (COUNTED = false).
 // A set far longer than a warp's share of a tile is cut into pieces taken by
-// several warps (ITEMS): 7.45 to 6.68 ms in the same case, 0.27 to 0.23 ms for
-// 7,056 states x 700 frames.
+// several warps (ITEMS): 7.45 to 6.68 ms in the same case, 0.29 to 0.23 ms for
+// 4,500 states x 1,003 frames.
 #include "rspi_common.cuh"
 
 namespace {
@@ -736,7 +736,9 @@ k_screen_sets(const float4 *__restrict__ lsl4, int num_rot, const double *__rest
             __syncthreads();   // every warp is done with the previous part
             tmem_fence_after();
             if (threadIdx.x == 0) {
-                next_set[0] = next_set[1] = next_set[2] = next_set[3] = 0;
+                // every warp's first set is its own place in its queue
+                for (int q = 0; q < 4; ++q)
+                    next_set[q] = ((int)(blockDim.x >> 5) - q + n_queues - 1) / n_queues;
                 const float4 *src = lsl4 + (t * n_parts + h) * (long long)part_w;
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar_a),
@@ -757,6 +759,47 @@ k_screen_sets(const float4 *__restrict__ lsl4, int num_rot, const double *__rest
                                      "r"(min(32768u, bytes - o))
                                      : "memory");
                 }
+            }
+            // the first set's range and entries, while the part is copied
+            // (72,900 states x 20,000 frames: 38.1 to 37.7 ms)
+            int s = 0, ng = 0, nq = 0;
+            unsigned piece = 0;
+            const uint2 *gp = groups;
+            uint2 c0 = make_uint2(0, 0), c1 = c0;
+            const int i_end = ITEMS ? item_off[h * n_queues + queue + 1] : n_sets;
+            auto take = [&](int i) {   // i-th of the queue; s < 0: no more
+                long long g0;
+                if (ITEMS) {
+                    i += item_off[h * n_queues + queue];
+                    s = -1;
+                    if (i >= i_end) return;
+                    const int4 *it = items + 2 * (long long)i;
+                    nq = reinterpret_cast<const int *>(it + 1)[lane >> 3];
+                    const int4 head = *it;
+                    s = head.x;
+                    g0 = head.y;
+                    ng = head.z;
+                    piece = (unsigned)head.w;
+                } else {
+                    s = queue + n_queues * i;
+                    if (s >= i_end) {
+                        s = -1;
+                        return;
+                    }
+                    const long long gi = (long long)h * n_sets + s;
+                    g0 = goff[gi];
+                    ng = (int)(goff[gi + 1] - g0);
+                    nq = qgroups ? qgroups[gi * 4 + (lane >> 3)] : ng;
+                }
+                // the set runs ng groups; this lane's quarter warp stops after
+                // its own nq (<= ng): its later gathers are not issued, so
+                // they take no shared-memory wavefront
+                gp = groups + g0 * 32 + lane;
+                c0 = 0 < nq ? ld_entries(gp, keep) : make_uint2(0, 0);
+                c1 = 1 < nq ? ld_entries(gp + 32, keep) : make_uint2(0, 0);
+            };
+            take(warp / n_queues);
+            if (threadIdx.x == 0) {
                 // bounded wait for the copy
                 const unsigned long long t0 = global_ns();
                 unsigned ready = 0;
@@ -799,39 +842,14 @@ k_screen_sets(const float4 *__restrict__ lsl4, int num_rot, const double *__rest
                 for (int k = 0; k < 4; ++k)
                     if (k < nt) ini[k] = init[(first + k) / num_rot];
             }
-            while (true) {
-                // set s from group g0 on: the warp runs ng groups; this lane's
-                // quarter warp stops after its own nq (<= ng): its later
-                // gathers are not issued, so they take no shared-memory
-                // wavefront
-                int s = 0, ng, nq;
-                long long g0;
-                unsigned piece = 0;
-                if (ITEMS) {
-                    if (lane == 0) s = atomicAdd(&next_set[queue], 1);
-                    s = __shfl_sync(RSPI_FULL_MASK, s, 0) + item_off[h * n_queues + queue];
-                    if (s >= item_off[h * n_queues + queue + 1]) break;
-                    const int4 *it = items + 2 * (long long)s;
-                    nq = reinterpret_cast<const int *>(it + 1)[lane >> 3];
-                    const int4 head = *it;
-                    s = head.x;
-                    g0 = head.y;
-                    ng = head.z;
-                    piece = (unsigned)head.w;
-                } else {
-                    if (lane == 0) s = queue + n_queues * atomicAdd(&next_set[queue], 1);
-                    s = __shfl_sync(RSPI_FULL_MASK, s, 0);
-                    if (s >= n_sets) break;
-                    const long long gi = (long long)h * n_sets + s;
-                    g0 = goff[gi];
-                    ng = (int)(goff[gi + 1] - g0);
-                    nq = qgroups ? qgroups[gi * 4 + (lane >> 3)] : ng;
-                }
+            auto next = [&]() {
+                int i = 0;
+                if (lane == 0) i = atomicAdd(&next_set[queue], 1);
+                take(__shfl_sync(RSPI_FULL_MASK, i, 0));
+            };
+            for (; s >= 0; next()) {
                 float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), a1 = a0;
-                const uint2 *gp = groups + g0 * 32 + lane;
                 int k = 0;
-                uint2 c0 = 0 < nq ? ld_entries(gp, keep) : make_uint2(0, 0);
-                uint2 c1 = 1 < nq ? ld_entries(gp + 32, keep) : make_uint2(0, 0);
                 for (; k + 1 < ng; k += 2, gp += 64) {
                     const uint2 n0 = k + 2 < nq ? ld_entries(gp + 64, keep) : make_uint2(0, 0);
                     const uint2 n1 = k + 3 < nq ? ld_entries(gp + 96, keep) : make_uint2(0, 0);
