@@ -614,11 +614,12 @@ int rspi_maxlp_pattern(double *fconv, const int *pixels, const int *hist_row,
                        long long size, int rescale_mode, const double *rescale,
                        int num_iter, double *rescale_out, cudaStream_t stream);
 
-/* rspi_maxlp_pattern with an FP32 screening pass per iteration: every
- * candidate is first evaluated in FP32 with a rigorous bound on its distance
- * from the FP64 value; only the candidates that can still be the argmax
- * (the finalists; every candidate without a finite bound) are evaluated in
- * FP64, with the same sums and roundings as rspi_maxlp_pattern, so the
+/* rspi_maxlp_pattern with a screening pass per iteration: every candidate's
+ * value is first bounded (a 3 x 3 cell around an FP32 value of its centre,
+ * then FP32 values of the survivors; or an order-8 expansion around f where
+ * the step is small against every f + r), rigorously against the FP64 value;
+ * only the candidates that can still be the argmax (the finalists; every
+ * candidate without a finite bound) are evaluated in FP64, with the same sums and roundings as rspi_maxlp_pattern, so the
  * chosen candidates, and fconv and rescale_out, are bit-identical to it.
  * Pixels with more than 1024 populated states, counts >= 2^24, or ring
  * pixels without photons run the FP64 iterations.  stats (device, 3
@@ -750,6 +751,12 @@ int rspi_rot_log_fixed(const double *holo, long long n_states0, long long num_ro
                        const int *sel_pix, long long n_sel, long long k_pad,
                        long long row_begin, long long row_end, long long plane_rows,
                        void *digits, int *err, cudaStream_t stream);
+/* The same from the pairs of rspi_holo_pairs (16-byte aligned). */
+int rspi_rot_log_fixed_pairs(const double *holo_pairs, long long n_states0, long long num_rot,
+                             const double *rot_cs, long long size, const double *bg,
+                             const int *sel_pix, long long n_sel, long long k_pad,
+                             long long row_begin, long long row_end, long long plane_rows,
+                             void *digits, int *err, cudaStream_t stream);
 
 int rspi_dense_loglike_i8(const void *a, const void *digits, long long k_pad,
                           long long n_frames, long long n_brows, long long num_rot,

@@ -430,14 +430,20 @@ __global__ void k_dense_frames_u8(const unsigned short *__restrict__ frames, lon
 // rint(L 2^21) as four 8-bit digit planes b[part][row][c] (zero beyond n_sel).
 // |L| is below 1024 for every value rot_log_value returns (the -1000 sentinel,
 // and logs of doubles); a larger value is clamped and flagged.
-// A CTA takes one rotation j and up to RQ_STATES consecutive states, a thread
-// four consecutive columns (one 32-bit store per digit plane): the columns'
-// rotated positions depend on (j, column) only and are computed once for the
-// states.  Bound by the FP64 pipe (interpolation and log): 9,720 rows x 47,616
-// columns 2.99 ms (3.25 with a row per CTA, positions computed per value).
+// A CTA takes one rotation j and up to RQ_STATES consecutive states, a warp
+// 128 columns, 32 neighbours at a time: the columns' rotated positions depend
+// on (j, column) only and are computed once for the states, and the four
+// digits of four lanes' columns change places (two shuffles) for one 32-bit
+// store per digit plane.  PAIRS: holo as (w[p], w[p + 1]) pairs, so that a
+// corner row is one 16-byte load.  Bound by L1 (75% of its wavefronts with
+// four columns of a thread side by side and 8-byte loads) and by issue; 9,720
+// rows x 47,616 columns: 3.25 ms with a row per CTA, 2.99 with eight states,
+// 2.87 with neighbouring columns, 2.67 with pairs and four CTAs per SM (three
+// 2.85, five 2.92; four states 2.81, sixteen 2.99).
 constexpr int RQ_STATES = 8;
 
-__global__ void __launch_bounds__(256)
+template <bool PAIRS>
+__global__ void __launch_bounds__(256, 4)
 k_rot_log_q(const double *__restrict__ holo, int num_rot, const double *__restrict__ rot_cs,
             int size, const double *__restrict__ bg, const int *__restrict__ sel_pix, int n_sel,
             int k_pad, long long row_begin, long long row_end, long long s_lo, long long plane,
@@ -453,15 +459,17 @@ k_rot_log_q(const double *__restrict__ holo, int num_rot, const double *__restri
     while (sb < se && sb * num_rot + j < row_begin) ++sb;
     while (se > sb && (se - 1) * num_rot + j >= row_end) --se;
     if (sb == se) return;
-    for (int c0 = 4 * threadIdx.x; c0 < k_pad; c0 += 4 * blockDim.x) {
+    const int lane = threadIdx.x & 31, i4 = lane & 3;
+    for (int cb = 4 * (threadIdx.x - lane); cb < k_pad; cb += 4 * blockDim.x) {
+        const int c0 = cb + lane;  // columns c0 + 32 u (k_pad is a multiple of 128)
         int at[4];                 // first corner; -1: outside the detector, -2: no column
         double fx[4], fy[4], bgv[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             at[u] = -2;
             fx[u] = fy[u] = bgv[u] = 0.;
-            if (c0 + u < n_sel) {
-                const int p = sel_pix[c0 + u];
+            if (c0 + 32 * u < n_sel) {
+                const int p = sel_pix[c0 + 32 * u];
                 int x, y;
                 pixel_xy(p, size, inv_size, x, y);
                 const double xc = (double)(x - cen), yc = (double)(y - cen);
@@ -476,17 +484,25 @@ k_rot_log_q(const double *__restrict__ holo, int num_rot, const double *__restri
             }
         }
         for (long long s0 = sb; s0 < se; ++s0) {
-            const double *w = holo + s0 * npix;
-            uint32_t dg[4] = {0u, 0u, 0u, 0u};
+            const double *w = holo + s0 * npix * (PAIRS ? 2 : 1);
             double t[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                const double *r0 = w + max(at[u], 0);
+                double2 r0, r1;
+                if (PAIRS) {
+                    const double2 *r = reinterpret_cast<const double2 *>(w) + max(at[u], 0);
+                    r0 = r[0];
+                    r1 = r[size];
+                } else {
+                    const double *r = w + max(at[u], 0);
+                    r0 = make_double2(r[0], r[1]);
+                    r1 = make_double2(r[size], r[size + 1]);
+                }
                 const double cx = 1. - fx[u], cy = 1. - fy[u];
-                double v = xmul(xmul(r0[0], cx), cy);
-                v = xadd(v, xmul(xmul(r0[size], fx[u]), cy));
-                v = xadd(v, xmul(xmul(r0[1], cx), fy[u]));
-                v = xadd(v, xmul(xmul(r0[size + 1], fx[u]), fy[u]));
+                double v = xmul(xmul(r0.x, cx), cy);
+                v = xadd(v, xmul(xmul(r1.x, fx[u]), cy));
+                v = xadd(v, xmul(xmul(r0.y, cx), fy[u]));
+                v = xadd(v, xmul(xmul(r1.y, fx[u]), fy[u]));
                 t[u] = xadd(v, bgv[u]);
             }
 #pragma unroll
@@ -497,14 +513,15 @@ k_rot_log_q(const double *__restrict__ holo, int num_rot, const double *__restri
                     rspi_flag(err, RSPI_ERR_CAPACITY);
                     v = v != v ? 0. : (v > 0. ? 1023. : -1023.);
                 }
-                const uint32_t q = (uint32_t)__double2int_rn(v * 2097152.);   // rint(v 2^21)
-#pragma unroll
-                for (int d = 0; d < 4; ++d) dg[d] |= ((q >> (8 * d)) & 255u) << (8 * u);
+                uint32_t q = (uint32_t)__double2int_rn(v * 2097152.);   // rint(v 2^21)
+                // digit bytes of four lanes' columns to the lane of their plane
+                const uint32_t a = __shfl_xor_sync(RSPI_FULL_MASK, q, 1);
+                q = __byte_perm(q, a, i4 & 1 ? 0x3715 : 0x6240);
+                const uint32_t e = __shfl_xor_sync(RSPI_FULL_MASK, q, 2);
+                q = __byte_perm(q, e, i4 & 2 ? 0x3276 : 0x5410);
+                *reinterpret_cast<uint32_t *>(b + (s0 * num_rot + j - row_begin) * (long long)k_pad +
+                                              i4 * plane + cb + 32 * u + lane - i4) = q;
             }
-            uint8_t *o = b + (s0 * num_rot + j - row_begin) * (long long)k_pad + c0;
-#pragma unroll
-            for (int d = 0; d < 4; ++d)
-                *reinterpret_cast<uint32_t *>(o + (long long)d * plane) = dg[d];
         }
     }
 }
@@ -638,11 +655,12 @@ extern "C" int rspi_dense_frames_u8(const unsigned short *frames, long long n_fr
     RSPI_RETURN_LAUNCH();
 }
 
-extern "C" int rspi_rot_log_fixed(const double *holo, long long n_states0, long long num_rot,
-                                  const double *rot_cs, long long size, const double *bg,
-                                  const int *sel_pix, long long n_sel, long long k_pad,
-                                  long long row_begin, long long row_end, long long plane_rows,
-                                  void *digits, int *err, cudaStream_t stream) {
+template <bool PAIRS>
+static int rot_log_fixed(const double *holo, long long n_states0, long long num_rot,
+                         const double *rot_cs, long long size, const double *bg,
+                         const int *sel_pix, long long n_sel, long long k_pad,
+                         long long row_begin, long long row_end, long long plane_rows,
+                         void *digits, int *err, cudaStream_t stream) {
     if (n_states0 <= 0 || num_rot <= 0 || size <= 1 || size > 46340 || k_pad < n_sel ||
         k_pad % 128 || row_begin < 0 || row_end > n_states0 * num_rot || row_end < row_begin ||
         plane_rows < row_end - row_begin || !holo || !rot_cs || !bg || !digits || !err ||
@@ -654,10 +672,30 @@ extern "C" int rspi_rot_log_fixed(const double *holo, long long n_states0, long 
     const long long blocks = ((s_hi - s_lo) / RQ_STATES + 1) * num_rot;
     if (blocks > 0x7fffffffLL || k_pad > 0x7fffffffLL || num_rot > 0x7fffffffLL)
         return RSPI_ERR_ARG;
-    k_rot_log_q<<<(unsigned)blocks, 256, 0, stream>>>(
+    k_rot_log_q<PAIRS><<<(unsigned)blocks, 256, 0, stream>>>(
         holo, (int)num_rot, rot_cs, (int)size, bg, sel_pix, (int)n_sel, (int)k_pad, row_begin,
         row_end, s_lo, plane_rows * k_pad, (uint8_t *)digits, err);
     RSPI_RETURN_LAUNCH();
+}
+
+extern "C" int rspi_rot_log_fixed(const double *holo, long long n_states0, long long num_rot,
+                                  const double *rot_cs, long long size, const double *bg,
+                                  const int *sel_pix, long long n_sel, long long k_pad,
+                                  long long row_begin, long long row_end, long long plane_rows,
+                                  void *digits, int *err, cudaStream_t stream) {
+    return rot_log_fixed<false>(holo, n_states0, num_rot, rot_cs, size, bg, sel_pix, n_sel,
+                                k_pad, row_begin, row_end, plane_rows, digits, err, stream);
+}
+
+extern "C" int rspi_rot_log_fixed_pairs(const double *holo_pairs, long long n_states0,
+                                        long long num_rot, const double *rot_cs, long long size,
+                                        const double *bg, const int *sel_pix, long long n_sel,
+                                        long long k_pad, long long row_begin, long long row_end,
+                                        long long plane_rows, void *digits, int *err,
+                                        cudaStream_t stream) {
+    if ((reinterpret_cast<uintptr_t>(holo_pairs) & 15) != 0) return RSPI_ERR_ARG;
+    return rot_log_fixed<true>(holo_pairs, n_states0, num_rot, rot_cs, size, bg, sel_pix, n_sel,
+                               k_pad, row_begin, row_end, plane_rows, digits, err, stream);
 }
 
 extern "C" int rspi_dense_loglike_i8(const void *a, const void *digits, long long k_pad,

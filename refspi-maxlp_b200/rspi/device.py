@@ -439,6 +439,7 @@ class EStep:
         self.vscale = torch.empty(1, dtype=_f64, device=dev)
         self.init = torch.empty(self.n_states0, dtype=_f64, device=dev)
         if gemm == 'i8':
+            self.holo_pairs = torch.empty((self.n_states0, npix, 2), dtype=_f64, device=dev)
             self.lsl = torch.empty((4, self.chunk_rows, self.k_pad), dtype=torch.uint8, device=dev)
         else:
             self.lsl_hi = torch.empty((self.chunk_rows, self.k_pad), dtype=torch.bfloat16,
@@ -742,7 +743,7 @@ class EStep:
                  self.n_sel, ptr(self.holo[g0]), ptr(self.msum[g0:]), s)
         call('rspi_vscale_init', ptr(self.msum), self.n_states0, ptr(self.ph.powder),
              ptr(self.sel_pix), self.n_sel, ptr(self.vscale), ptr(self.init), s)
-        if self.form != 'dense':
+        if self.form != 'dense' or self.dense_gemm == 'i8':
             call('rspi_holo_pairs', ptr(self.holo), self.n_states0, self.size,
                  ptr(self.holo_pairs), s)
         if self.form != 'fp64':
@@ -758,7 +759,7 @@ class EStep:
     def rot_slices(self, r0, r1, out=None):
         """a6: rotated log-slices of rows [r0, r1) into ``out`` (or the chunk buffer)."""
         if self.form == 'dense' and self.dense_gemm == 'i8':
-            call('rspi_rot_log_fixed', ptr(self.holo), self.n_states0, self.num_rot,
+            call('rspi_rot_log_fixed_pairs', ptr(self.holo_pairs), self.n_states0, self.num_rot,
                  ptr(self.rot_cs), self.size, ptr(self.bg), ptr(self.sel_pix), self.n_sel,
                  self.k_pad, r0, r1, self.chunk_rows, ptr(self.lsl), ptr(self.ph.err.t),
                  cur_stream())
@@ -1002,8 +1003,9 @@ class MStep:
     over the frames assigned to it, with its own ring rescale, in the same
     launches.
 
-    ``screen`` (default): each pattern iteration evaluates every candidate in
-    FP32 with a rigorous error bound and only the finalists in FP64; the
+    ``screen`` (default): each pattern iteration bounds every candidate's
+    value (cells of nine, or an expansion around the pixel's value, then FP32
+    values) and evaluates only the finalists in FP64; the
     chosen candidates are bit-identical to ``screen=False`` (every candidate
     in FP64).  ``stats`` (device int64[3]) counts the iterations the screen
     settled, the iterations that ran the FP64 pass, and the finalists."""

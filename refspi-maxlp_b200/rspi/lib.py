@@ -104,6 +104,7 @@ SIGNATURES = {
     'rspi_maxlp_grid': (I, [P, P, P, L, P, L, P, P, L, P, L, I, I, P, P, P, P]),
     'rspi_dense_frames_u8': (I, [P, L, L, P, L, L, P, P, P]),
     'rspi_rot_log_fixed': (I, [P, L, L, P, L, P, P, L, L, L, L, L, P, P, P]),
+    'rspi_rot_log_fixed_pairs': (I, [P, L, L, P, L, P, P, L, L, L, L, L, P, P, P]),
     'rspi_dense_loglike_i8': (I, [P, P, L, L, L, L, L, L, P, P, P, L, P, P]),
 }
 
@@ -162,7 +163,7 @@ KERNELS_PER_CALL = {
     'rspi_screen_loglike_sets': 1, 'rspi_frame_max_finalize': 1,
     'rspi_screen_candidates_cols': 4, 'rspi_rescore_cols': 5, 'rspi_nll': 2, 'rspi_nll_grid': 2, 'rspi_screen_candidates_noalloc': 3, 'rspi_merge_coverage': 1, 'rspi_merge': 2, 'rspi_merge_rows': 2,
     'rspi_dense_frames': 1, 'rspi_rot_log_split': 1, 'rspi_dense_loglike': 1,
-    'rspi_maxlp_grid': 2, 'rspi_dense_frames_u8': 1, 'rspi_rot_log_fixed': 1,
+    'rspi_maxlp_grid': 2, 'rspi_dense_frames_u8': 1, 'rspi_rot_log_fixed': 1, 'rspi_rot_log_fixed_pairs': 1,
     'rspi_dense_loglike_i8': 1, 'rspi_sets_entries_check': 1, 'rspi_sim_views': 1, 'rspi_sim_counts': 1,
     'rspi_sim_poisson': 1, 'rspi_sim_sparse_counts': 1, 'rspi_sim_sparse_fill': 1,
 }
