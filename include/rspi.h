@@ -532,17 +532,20 @@ int rspi_merge(const int *pair_d, const int *pair_r, const double *pair_ll,
                cudaStream_t stream);
 
 /* rspi_merge with the pairs grouped by likelihood row, as rspi_rescore leaves
- * the candidates: row r's pairs are row_cand[row_off[r] .. row_off[r + 1]).
+ * the candidates: row r's pairs are row_cand[row_off[r] .. row_off[r + 1]),
+ * pair_r their rows, row_off[n_rows] their number; row_done: n_rows ints of
+ * scratch.
  * `images` holds n_images scratch images of size^2 doubles, one per CTA (two
  * per SM).  Sums differ from rspi_merge's by their FP64 rounding. */
-int rspi_merge_rows(const int *pair_d, const double *pair_ll, const long long *row_off,
-                    const int *row_cand, const double *logz, double p_min,
-                    const double *scales, const int *ones, const int *multi,
+int rspi_merge_rows(const int *pair_d, const int *pair_r, const double *pair_ll,
+                    const long long *row_off, const int *row_cand, const double *logz,
+                    double p_min, const double *scales, const int *ones, const int *multi,
                     const long long *ones_accum, const long long *multi_accum,
                     const int *place_ones, const int *place_multi, const int *count_multi,
                     long long n_states0, long long num_rot, const double *rot_cs,
                     long long size, const double *cov, double *num, double *den, double *w,
-                    double *intens, double *images, long long n_images, cudaStream_t stream);
+                    double *intens, int *row_done, double *images, long long n_images,
+                    cudaStream_t stream);
 
 /* ----------------------------------------------------------------- a11-a14
  * MaxLP M-step (maxLP.py:304-340).  Frames carry a reference-state index

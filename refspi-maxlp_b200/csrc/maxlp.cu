@@ -813,7 +813,7 @@ k_pattern_screen(double2 *__restrict__ fconv, const int *__restrict__ pixels,
         if (h > 0) r = make_double2(re[s], im[s]);
         const unsigned bal = __ballot_sync(RSPI_FULL_MASK, h > 0);
         if (lane == 0) wsum[wid] = __popc(bal);
-        __syncthreads();   // counts in place; this round's r are in registers
+        __syncthreads();   // counts in place; this turn's r are in registers
         int before = 0, round = 0;
 #pragma unroll
         for (int w = 0; w < PS_WARPS; ++w) {

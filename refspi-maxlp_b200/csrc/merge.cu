@@ -95,7 +95,8 @@ __device__ __forceinline__ void scatter4(double *__restrict__ acc, int size, int
 }
 
 // One warp per significant pair: scatter P * K_d back through rotation j
-// into num[s0] and add P * scale_d to w[r].
+// into num[s0] and add P * scale_d to w[r].  With row_done only the pairs of
+// rows that k_merge_rows left.  A warp tests up to eight pairs at once.
 __global__ void __launch_bounds__(256)
 k_merge_scatter(const int *__restrict__ pd, const int *__restrict__ pr,
                 const double *__restrict__ pll, const long long *__restrict__ total_ptr,
@@ -105,51 +106,71 @@ k_merge_scatter(const int *__restrict__ pd, const int *__restrict__ pr,
                 const long long *__restrict__ multi_accum, const int *__restrict__ place_ones,
                 const int *__restrict__ place_multi, const int *__restrict__ count_multi,
                 long long num_rot, const double *__restrict__ rot_cs, int size,
-                double *__restrict__ num, double *__restrict__ w) {
+                const int *__restrict__ row_done, double *__restrict__ num,
+                double *__restrict__ w) {
     const int lane = threadIdx.x & 31;
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nwarp = ((long long)gridDim.x * blockDim.x) >> 5;
     const long long total = min(*total_ptr, capacity);
     const long long npix = (long long)size * size;
-    for (long long i = warp; i < total; i += nwarp) {
-        const int d = pd[i], r = pr[i];
-        const double p = exp(pll[i] - logz[d]);
-        if (!(p >= p_min)) continue;
-        const long long s0 = r / num_rot, j = r - s0 * num_rot;
-        const double ac = rot_cs[2 * j], as = rot_cs[2 * j + 1];
-        double *acc = num + s0 * npix;
-        if (lane == 0) atomicAdd(&w[r], p * scales[d]);
-        const int n_o = ones[d], n_m = multi[d];
-        const long long oa = ones_accum[d], ma = multi_accum[d];
-        for (int k = lane; k < n_o + n_m; k += 32) {
-            int pix;
-            double cnt;
-            if (k < n_o) {
-                pix = place_ones[oa + k];
-                cnt = 1.;
-            } else {
-                pix = place_multi[ma + k - n_o];
-                cnt = (double)count_multi[ma + k - n_o];
+    const int per = (int)max(1LL, min(8LL, (total + nwarp - 1) / nwarp));
+    for (long long i0 = warp * per; i0 < total; i0 += nwarp * per) {
+        int my_d = 0, my_r = 0;
+        double my_p = 0.;
+        bool mine = lane < per && i0 + lane < total;
+        if (mine) {
+            my_r = pr[i0 + lane];
+            mine = !row_done || !row_done[my_r];
+        }
+        if (mine) {
+            my_d = pd[i0 + lane];
+            my_p = exp(pll[i0 + lane] - logz[my_d]);
+            mine = my_p >= p_min;
+        }
+        for (unsigned left = __ballot_sync(RSPI_FULL_MASK, mine); left; left &= left - 1) {
+            const int src = __ffs(left) - 1;
+            const int d = __shfl_sync(RSPI_FULL_MASK, my_d, src);
+            const int r = __shfl_sync(RSPI_FULL_MASK, my_r, src);
+            const double p = __shfl_sync(RSPI_FULL_MASK, my_p, src);
+            const long long s0 = r / num_rot, j = r - s0 * num_rot;
+            const double ac = rot_cs[2 * j], as = rot_cs[2 * j + 1];
+            double *acc = num + s0 * npix;
+            if (lane == 0) atomicAdd(&w[r], p * scales[d]);
+            const int n_o = ones[d], n_m = multi[d];
+            const long long oa = ones_accum[d], ma = multi_accum[d];
+            for (int k = lane; k < n_o + n_m; k += 32) {
+                int pix;
+                double cnt;
+                if (k < n_o) {
+                    pix = place_ones[oa + k];
+                    cnt = 1.;
+                } else {
+                    pix = place_multi[ma + k - n_o];
+                    cnt = (double)count_multi[ma + k - n_o];
+                }
+                if (pix < 0 || pix >= npix) continue;
+                int ix, iy;
+                double fx, fy;
+                if (footprint(pix / size, pix % size, size, ac, as, ix, iy, fx, fy))
+                    scatter4(acc, size, ix, iy, fx, fy, p * cnt);
             }
-            if (pix < 0 || pix >= npix) continue;
-            int ix, iy;
-            double fx, fy;
-            if (footprint(pix / size, pix % size, size, ac, as, ix, iy, fx, fy))
-                scatter4(acc, size, ix, iy, fx, fy, p * cnt);
         }
     }
 }
 
-// The same scatter with the pairs grouped by likelihood row, a CTA per row.
-// R_j^T is linear, so a row whose pairs hold many photons first sums P K_d
-// unrotated into the CTA's image (one FP64 reduction per photon) and then
-// turns that image back (four per populated pixel) instead of four per photon;
-// a row with fewer than npix / MR_DENSE photons scatters them directly.  The
-// reductions in L2 bound both: 848,000 pairs of 1,003 frames over 4,500 rows
-// of 185^2 (190 pairs a row) take 2.08 ms with two CTAs per SM (2.56 with one),
-// 3.75 with every photon turned.
+// The pairs of a likelihood row with many photons, a CTA per row.  R_j^T is
+// linear, so the row sums P K_d unrotated into the CTA's image (one FP64
+// reduction per photon) and then turns that image back (four per populated
+// pixel) instead of four per photon.  Rows with fewer than npix / MR_DENSE
+// photons are left to k_merge_scatter (row_done 0), which spreads them over
+// the GPU: the warps of a CTA would meet in the same pixels of one state.
+// The reductions in L2 bound both.  848,000 pairs of 1,003 frames over 4,500
+// rows of 185^2 take 1.98 ms with two CTAs per SM (2.56 with one), 3.75 with
+// every photon turned; 101,000 pairs of 1,138 frames over 4,400 rows of 174^2,
+// three of them dense, 0.77 ms by the scatter and 1.07 by row.
 constexpr int MR_THREADS = 1024;
 constexpr int MR_DENSE = 2;
+constexpr int MR_MIN_PAIRS = 16;   // a row's pairs before its photons are counted
 
 __global__ void __launch_bounds__(MR_THREADS, 2)
 k_merge_rows(const int *__restrict__ pd, const double *__restrict__ pll,
@@ -160,15 +181,30 @@ k_merge_rows(const int *__restrict__ pd, const double *__restrict__ pll,
              const long long *__restrict__ multi_accum, const int *__restrict__ place_ones,
              const int *__restrict__ place_multi, const int *__restrict__ count_multi,
              long long num_rot, const double *__restrict__ rot_cs, int size,
-             double *__restrict__ num, double *__restrict__ w, double *__restrict__ images) {
+             double *__restrict__ num, double *__restrict__ w, int *__restrict__ row_done,
+             double *__restrict__ images) {
     __shared__ double wsum[MR_THREADS / 32];
     __shared__ unsigned long long n_phot;
+    __shared__ int list[MR_THREADS], n_list;
+    __shared__ int sig_d[MR_THREADS], n_sig;   // significant pairs of a batch
+    __shared__ double sig_p[MR_THREADS];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int npix = size * size;
     double *view = images + (long long)blockIdx.x * npix;
-    for (long long r = blockIdx.x; r < n_rows; r += gridDim.x) {
+    // the CTA's rows r = blockIdx.x + k gridDim.x, tested MR_THREADS at a time
+    for (long long base = blockIdx.x; base < n_rows; base += (long long)gridDim.x * MR_THREADS) {
+    __syncthreads();   // the previous list's readers are done
+    if (threadIdx.x == 0) n_list = 0;
+    __syncthreads();
+    const long long rt = base + (long long)threadIdx.x * gridDim.x;
+    if (rt < n_rows) {
+        row_done[rt] = 0;
+        if (row_off[rt + 1] - row_off[rt] >= MR_MIN_PAIRS) list[atomicAdd(&n_list, 1)] = (int)rt;
+    }
+    __syncthreads();
+    for (int kr = 0; kr < n_list; ++kr) {
+        const long long r = list[kr];
         const long long a = row_off[r], b = row_off[r + 1];
-        if (a == b) continue;
         const long long s0 = r / num_rot, j = r - s0 * num_rot;
         const double ac = rot_cs[2 * j], as = rot_cs[2 * j + 1];
         double *acc = num + s0 * npix;
@@ -192,43 +228,51 @@ k_merge_rows(const int *__restrict__ pd, const double *__restrict__ pll,
             if (np) atomicAdd(&n_phot, (unsigned long long)np);
         }
         __syncthreads();
+        if (n_phot * MR_DENSE < (unsigned long long)npix) continue;
         if (threadIdx.x == 0) {
             double t = 0.;
             for (int k = 0; k < MR_THREADS / 32; ++k) t += wsum[k];
             w[r] = t;
+            row_done[r] = 1;
         }
-        const bool dense = n_phot * MR_DENSE >= (unsigned long long)npix;
-        if (dense) {
-            for (int t = threadIdx.x; t < npix; t += MR_THREADS) __stcg(view + t, 0.);
-            __threadfence();
+        for (int t = threadIdx.x; t < npix; t += MR_THREADS) __stcg(view + t, 0.);
+        __threadfence();
+        // a thread tests a pair (most of a row's may be below p_min); the warps
+        // share those that are not, several to a pair when they are few
+        for (long long i0 = a; i0 < b; i0 += MR_THREADS) {
+            __syncthreads();   // the previous batch's readers are done
+            if (threadIdx.x == 0) n_sig = 0;
             __syncthreads();
-        }
-        for (long long i = a + wid; i < b; i += MR_THREADS / 32) {   // a warp per pair
-            const int pair = row_cand[i], d = pd[pair];
-            const double p = exp(pll[pair] - logz[d]);
-            if (!(p >= p_min)) continue;
-            const int n_o = ones[d], n_m = multi[d];
-            const long long oa = ones_accum[d], ma = multi_accum[d];
-            for (int k = lane; k < n_o + n_m; k += 32) {
-                int pix;
-                double cnt;
-                if (k < n_o) {
-                    pix = place_ones[oa + k];
-                    cnt = 1.;
-                } else {
-                    pix = place_multi[ma + k - n_o];
-                    cnt = (double)count_multi[ma + k - n_o];
+            if (i0 + threadIdx.x < b) {
+                const int pair = row_cand[i0 + threadIdx.x], d = pd[pair];
+                const double p = exp(pll[pair] - logz[d]);
+                if (p >= p_min) {
+                    const int k = atomicAdd(&n_sig, 1);
+                    sig_d[k] = d;
+                    sig_p[k] = p;
                 }
-                if (pix < 0 || pix >= npix) continue;
-                int ix, iy;
-                double fx, fy;
-                if (dense)
-                    atomicAdd(view + pix, p * cnt);
-                else if (footprint(pix / size, pix % size, size, ac, as, ix, iy, fx, fy))
-                    scatter4(acc, size, ix, iy, fx, fy, p * cnt);
+            }
+            __syncthreads();
+            const int share = n_sig > 0 ? max(1, MR_THREADS / 32 / n_sig) : 1;
+            for (int q = wid / share; q < n_sig; q += MR_THREADS / 32 / share) {
+                const int d = sig_d[q];
+                const double p = sig_p[q];
+                const int n_o = ones[d], n_m = multi[d];
+                const long long oa = ones_accum[d], ma = multi_accum[d];
+                for (int k = lane + 32 * (wid % share); k < n_o + n_m; k += 32 * share) {
+                    int pix;
+                    double cnt;
+                    if (k < n_o) {
+                        pix = place_ones[oa + k];
+                        cnt = 1.;
+                    } else {
+                        pix = place_multi[ma + k - n_o];
+                        cnt = (double)count_multi[ma + k - n_o];
+                    }
+                    if (pix >= 0 && pix < npix) atomicAdd(view + pix, p * cnt);
+                }
             }
         }
-        if (!dense) continue;
         __threadfence();
         __syncthreads();   // the image is complete (in L2)
         for (int t = threadIdx.x; t < npix; t += MR_THREADS) {
@@ -239,6 +283,7 @@ k_merge_rows(const int *__restrict__ pd, const double *__restrict__ pll,
             if (footprint(t / size, t % size, size, ac, as, ix, iy, fx, fy))
                 scatter4(acc, size, ix, iy, fx, fy, v);
         }
+    }
     }
 }
 
@@ -323,13 +368,13 @@ extern "C" int rspi_merge(const int *pair_d, const int *pair_r, const double *pa
     k_merge_scatter<<<rspi_sm_count() * 8, 256, 0, stream>>>(
         pair_d, pair_r, pair_ll, pair_total, capacity, logz, p_min, scales, ones, multi,
         ones_accum, multi_accum, place_ones, place_multi, count_multi, num_rot, rot_cs,
-        (int)size, num, w);
+        (int)size, nullptr, num, w);
     k_merge_finalize<<<rspi_blocks(n_states0 * npix, 256, 16), 256, 0, stream>>>(
         num, w, cov, n_states0, num_rot, npix, den, intens);
     RSPI_RETURN_LAUNCH();
 }
 
-extern "C" int rspi_merge_rows(const int *pair_d, const double *pair_ll,
+extern "C" int rspi_merge_rows(const int *pair_d, const int *pair_r, const double *pair_ll,
                                const long long *row_off, const int *row_cand, const double *logz,
                                double p_min, const double *scales, const int *ones,
                                const int *multi, const long long *ones_accum,
@@ -337,11 +382,11 @@ extern "C" int rspi_merge_rows(const int *pair_d, const double *pair_ll,
                                const int *place_multi, const int *count_multi,
                                long long n_states0, long long num_rot, const double *rot_cs,
                                long long size, const double *cov, double *num, double *den,
-                               double *w, double *intens, double *images, long long n_images,
-                               cudaStream_t stream) {
-    if (!pair_d || !pair_ll || !row_off || !row_cand || !logz || !scales || !ones || !multi ||
+                               double *w, double *intens, int *row_done, double *images,
+                               long long n_images, cudaStream_t stream) {
+    if (!pair_d || !pair_r || !pair_ll || !row_off || !row_cand || !logz || !scales || !ones || !multi ||
         !ones_accum || !multi_accum || !rot_cs || !cov || !num || !den || !w || !intens ||
-        !images || n_images < 1 || n_states0 <= 0 || num_rot <= 0 || size <= 1 || size > 46340)
+        !row_done || !images || n_images < 1 || n_states0 <= 0 || num_rot <= 0 || size <= 1 || size > 46340)
         return RSPI_ERR_ARG;
     const long long npix = size * size, n_rows = n_states0 * num_rot;
     cudaMemsetAsync(num, 0, sizeof(double) * n_states0 * npix, stream);
@@ -350,7 +395,11 @@ extern "C" int rspi_merge_rows(const int *pair_d, const double *pair_ll,
     k_merge_rows<<<grid, MR_THREADS, 0, stream>>>(
         pair_d, pair_ll, row_off, row_cand, n_rows, logz, p_min, scales, ones, multi, ones_accum,
         multi_accum, place_ones, place_multi, count_multi, num_rot, rot_cs, (int)size, num, w,
-        images);
+        row_done, images);
+    k_merge_scatter<<<rspi_sm_count() * 8, 256, 0, stream>>>(
+        pair_d, pair_r, pair_ll, row_off + n_rows, 0x7fffffffLL, logz, p_min, scales, ones, multi,
+        ones_accum, multi_accum, place_ones, place_multi, count_multi, num_rot, rot_cs, (int)size,
+        row_done, num, w);
     k_merge_finalize<<<rspi_blocks(n_states0 * npix, 256, 16), 256, 0, stream>>>(
         num, w, cov, n_states0, num_rot, npix, den, intens);
     RSPI_RETURN_LAUNCH();

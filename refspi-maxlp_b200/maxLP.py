@@ -8,9 +8,9 @@ constructor and ``_run_phaser(model, sx_vals, sy_vals, dia_vals, ang_vals)``
 ``get_fref_d``, ``get_pixel_constants``, ``get_rescale_pixel``,
 ``get_logq_pixel``, ``iterate_pixel_pattern``, ``run_pixel_pattern``,
 ``_get_sphere``, ``get_fcalc_all``), all on the device.  The per-pixel
-pattern search runs in librspi (one CTA per pixel, all 1089 candidates at
-once); see csrc/maxlp.cu for the exact sparse/analytic rewrite of
-``get_logq_pixel``.
+pattern search runs in librspi (one CTA per pixel; candidates bounded in
+cells or by an expansion, the finalists in FP64); see csrc/maxlp.cu for the
+exact sparse/analytic rewrite of ``get_logq_pixel``.
 """
 import os
 import sys

@@ -589,8 +589,8 @@ class EStep:
             call('rspi_sets_counts32', ptr(ll['entries']), ptr(ll['row_off']), n, pz, parts,
                  part_w, ptr(counts), s)
             tot = counts.view(n, 32).sum(1)
-            phot = ll['frame_sel_photons'].sum()
-            counted = bool((COUNT_GAIN * (phot - tot.sum()) >= phot).item())
+            phot = int(ll['frame_sel_photons'].sum())
+            counted = COUNT_GAIN * (phot - int(tot.sum())) >= phot
         if not counted:
             ll = self.ll16
             call('rspi_sets_counts', ptr(ll['entries']), ptr(ll['row_off']), n, pz, parts, part_w,
@@ -661,35 +661,33 @@ class EStep:
         set of a part, or, of the first SPLIT_SETS sets, an even piece of one
         longer than SPLIT_SHARES warps' shares of the part's groups.  Returns
         (items, item_off, seg_slots), (None, None, 0) when no set is cut."""
-        dev = groups.device
-        g = groups.view(parts, n_sets).to(_i64)
-        share = (g.sum(1, keepdim=True) // SPLIT_WARPS).clamp(min=1)
-        s = torch.arange(n_sets, device=dev)
-        n_seg = torch.where((s < SPLIT_SETS) & (g > SPLIT_SHARES * share),
-                            (g + share - 1) // share, 1).clamp(max=127)
-        queues = 4 if parts > 1 else 1
-        pos = torch.argsort(s % queues, stable=True)      # sets queue by queue
-        at = (torch.arange(parts, device=dev)[:, None] * n_sets + pos).view(-1)
-        g, n_seg = g.view(-1), n_seg.view(parts, n_sets)
-        split = torch.where(n_seg > 1, n_seg, 0)
-        base = (split.cumsum(1) - split).view(-1)
-        off = torch.zeros(parts * queues + 1, dtype=_i64, device=dev)
-        off[1:] = torch.stack([n_seg[:, q::queues].sum(1) for q in range(queues)],
-                              1).view(-1).cumsum(0)
-        n_seg = n_seg.view(-1)
-        n_items, slots = torch.stack([off[-1], split.sum(1).max()]).tolist()
+        g = groups.cpu().numpy().reshape(parts, n_sets).astype(np.int64)
+        share = np.maximum(g.sum(1, keepdims=True) // SPLIT_WARPS, 1)
+        n_seg = np.where((np.arange(n_sets) < SPLIT_SETS) & (g > SPLIT_SHARES * share),
+                         np.minimum((g + share - 1) // share, 127), 1)
+        split = np.where(n_seg > 1, n_seg, 0)
+        slots = int(split.sum(1).max())
         if slots == 0:
             return None, None, 0
-        rep = torch.repeat_interleave(at, n_seg[at], output_size=n_items)
-        first = n_seg[at].cumsum(0) - n_seg[at]
-        k = torch.arange(n_items, device=dev) - \
-            torch.repeat_interleave(first, n_seg[at], output_size=n_items)
+        queues = 4 if parts > 1 else 1
+        off = np.zeros(parts * queues + 1, np.int64)
+        off[1:] = np.stack([n_seg[:, q::queues].sum(1) for q in range(queues)], 1).cumsum()
+        base = (split.cumsum(1) - split).ravel()
+        pos = np.argsort(np.arange(n_sets) % queues, kind='stable')   # sets queue by queue
+        at = (np.arange(parts)[:, None] * n_sets + pos).ravel()
+        g, n_seg = g.ravel(), n_seg.ravel()
+        rep = np.repeat(at, n_seg[at])
+        k = np.arange(rep.size) - np.repeat(n_seg[at].cumsum() - n_seg[at], n_seg[at])
         k0, k1 = g[rep] * k // n_seg[rep], g[rep] * (k + 1) // n_seg[rep]
-        quarters = qgroups.view(-1, 4)[rep].to(_i64) - k0[:, None]
-        quarters = torch.minimum(quarters.clamp(min=0), (k1 - k0)[:, None])
-        items = torch.cat([torch.stack([rep % n_sets, goff[rep] + k0, k1 - k0,
-                                        base[rep] | k << 16 | n_seg[rep] << 24], 1), quarters], 1)
-        return items.to(_i32).contiguous(), off.to(_i32), slots
+        quarters = qgroups.cpu().numpy().reshape(-1, 4)[rep].astype(np.int64) - k0[:, None]
+        items = np.empty((rep.size, 8), np.int32)
+        items[:, 0] = rep % n_sets
+        items[:, 1] = goff.cpu().numpy()[rep] + k0
+        items[:, 2] = k1 - k0
+        items[:, 3] = base[rep] | k << 16 | n_seg[rep] << 24
+        items[:, 4:] = np.clip(quarters, 0, (k1 - k0)[:, None])
+        return (torch.from_numpy(items).to(groups.device),
+                torch.from_numpy(off.astype(np.int32)).to(groups.device), slots)
 
     def _eps_rows(self):
         """Prefix sums of each frame's FP32 summation length for the
@@ -950,6 +948,7 @@ class Merge:
             # an unrotated image per CTA of the row-grouped scatter, two per SM
             sms = torch.cuda.get_device_properties(dev).multi_processor_count
             self.images = torch.empty((2 * sms, npix), dtype=_f64, device=dev)
+            self.row_done = torch.empty(estep.n_rows, dtype=_i32, device=dev)
         else:
             self.cnt_part = torch.empty(n * 32, dtype=_i32, device=dev)
             self.cnt = torch.empty(n, dtype=_i32, device=dev)
@@ -979,12 +978,13 @@ class Merge:
                 self._alloc(int(total * 1.25) + 1024)
         else:
             # the rescoring left the candidates grouped by likelihood row
-            call('rspi_merge_rows', ptr(es.cand_d), ptr(es.cand_ll), ptr(es.row_cand_off),
-                 ptr(es.row_cand), ptr(es.logz), self.p_min, ptr(ph.scales), ptr(ph.ones),
+            call('rspi_merge_rows', ptr(es.cand_d), ptr(es.cand_r), ptr(es.cand_ll),
+                 ptr(es.row_cand_off), ptr(es.row_cand), ptr(es.logz), self.p_min, ptr(ph.scales), ptr(ph.ones),
                  ptr(ph.multi), ptr(ph.ones_accum), ptr(ph.multi_accum), ptr(ph.place_ones),
                  ptr(ph.place_multi), ptr(ph.count_multi), es.n_states0, es.num_rot,
                  ptr(es.rot_cs), es.size, ptr(self.cov), ptr(self.num), ptr(self.den),
-                 ptr(self.w), ptr(self.intens), ptr(self.images), self.images.shape[0], s)
+                 ptr(self.w), ptr(self.intens), ptr(self.row_done), ptr(self.images),
+                 self.images.shape[0], s)
             return self.intens
         pd, pr, pll, tot, cap = self.pd, self.pr, self.pll, self.off[n:], self.capacity
         call('rspi_merge', ptr(pd), ptr(pr), ptr(pll), ptr(tot), cap, ptr(es.logz), self.p_min,

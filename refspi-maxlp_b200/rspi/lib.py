@@ -97,7 +97,7 @@ SIGNATURES = {
     'rspi_posterior_pairs': (I, [P, L, L, P, D, P, P, P, L, P, P, P, P, P]),
     'rspi_merge_coverage': (I, [L, P, L, P, P]),
     'rspi_merge': (I, [P, P, P, P, L, P, D, P, P, P, P, P, P, P, P, L, L, P, L, P, P, P, P, P, P]),
-    'rspi_merge_rows': (I, [P] * 5 + [D] + [P] * 8 + [L, L, P, L] + [P] * 6 + [L, P]),
+    'rspi_merge_rows': (I, [P] * 6 + [D] + [P] * 8 + [L, L, P, L] + [P] * 7 + [L, P]),
     'rspi_dense_frames': (I, [P, L, L, P, L, L, P, P, P, P]),
     'rspi_rot_log_split': (I, [P, L, L, P, L, P, P, L, L, L, L, P, P, P, P]),
     'rspi_dense_loglike': (I, [P, P, P, P, L, L, L, L, L, L, P, P, P, L, P, P]),
@@ -161,7 +161,7 @@ KERNELS_PER_CALL = {
     'rspi_screen_loglike_items': 1,
     'rspi_rot_log_slices_sets': 1, 'rspi_holo_quads32': 1, 'rspi_sets_part_sums_floats': 0,
     'rspi_screen_loglike_sets': 1, 'rspi_frame_max_finalize': 1,
-    'rspi_screen_candidates_cols': 4, 'rspi_rescore_cols': 5, 'rspi_nll': 2, 'rspi_nll_grid': 2, 'rspi_screen_candidates_noalloc': 3, 'rspi_merge_coverage': 1, 'rspi_merge': 2, 'rspi_merge_rows': 2,
+    'rspi_screen_candidates_cols': 4, 'rspi_rescore_cols': 5, 'rspi_nll': 2, 'rspi_nll_grid': 2, 'rspi_screen_candidates_noalloc': 3, 'rspi_merge_coverage': 1, 'rspi_merge': 2, 'rspi_merge_rows': 3,
     'rspi_dense_frames': 1, 'rspi_rot_log_split': 1, 'rspi_dense_loglike': 1,
     'rspi_maxlp_grid': 2, 'rspi_dense_frames_u8': 1, 'rspi_rot_log_fixed': 1, 'rspi_rot_log_fixed_pairs': 1,
     'rspi_dense_loglike_i8': 1, 'rspi_sets_entries_check': 1, 'rspi_sim_views': 1, 'rspi_sim_counts': 1,
