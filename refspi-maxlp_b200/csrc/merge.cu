@@ -165,9 +165,9 @@ k_merge_scatter(const int *__restrict__ pd, const int *__restrict__ pr,
 // photons are left to k_merge_scatter (row_done 0), which spreads them over
 // the GPU: the warps of a CTA would meet in the same pixels of one state.
 // The reductions in L2 bound both.  848,000 pairs of 1,003 frames over 4,500
-// rows of 185^2 take 1.98 ms with two CTAs per SM (2.56 with one), 3.75 with
-// every photon turned; 101,000 pairs of 1,138 frames over 4,400 rows of 174^2,
-// three of them dense, 0.77 ms by the scatter and 1.07 by row.
+// rows of 185^2 take 1.88 ms, both kernels (1.95 with every row here, 2.56 with
+// one CTA per SM, 3.75 with every photon turned); 101,000 pairs of 1,138 frames over 4,400 rows of 174^2,
+// three of them dense, 0.73 ms by the scatter and 1.07 by row.
 constexpr int MR_THREADS = 1024;
 constexpr int MR_DENSE = 2;
 constexpr int MR_MIN_PAIRS = 16;   // a row's pairs before its photons are counted
