@@ -244,8 +244,9 @@ int launch_dense(const GridTables &g, long long n_pix, int size, const double *f
                                                          gdia, gsx, gsy, gscale);
         return RSPI_OK;
     }
-    return launch_dense_grid<CT, GRAD>(g, n_pix, size, fre, fim, 1, 1., 0., dia, sx, sy, scale,
-                                       n_frames, out, gfre, gfim, gdia, gsx, gsy, gscale, stream);
+    return launch_dense_grid<CT, GRAD>(g, n_pix, size, fre, fim, 1, 1., 0., false, dia, sx, sy,
+                                       scale, n_frames, out, gfre, gfim, gdia, gsx, gsy, gscale,
+                                       stream);
 }
 
 template <typename CT, bool GRAD>

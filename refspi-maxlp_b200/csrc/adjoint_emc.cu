@@ -280,8 +280,8 @@ int emc_launch(const GridTables &g, double bg_sum, const double2 *model, int siz
                 double *gscale, int *err, cudaStream_t stream) {
     if (g.order) {
         const double *m = reinterpret_cast<const double *>(model);
-        const int st = launch_dense_grid<CT, GRAD>(g, n_sel, size, m, m + 1, 2, vscale, bg_sum, dia,
-                                                   sx, sy, scale, n_frames, out, gre, gim, gdia,
+        const int st = launch_dense_grid<CT, GRAD>(g, n_sel, size, m, m + 1, 2, vscale, bg_sum, true,
+                                                   dia, sx, sy, scale, n_frames, out, gre, gim, gdia,
                                                    gsx, gsy, gscale, stream);
         if (st != RSPI_OK) return st;
     } else if (n_sel > 0) {

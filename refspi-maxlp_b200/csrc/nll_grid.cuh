@@ -78,8 +78,9 @@ k_nll_dense_grid(const double *__restrict__ fre, const double *__restrict__ fim,
                  const int *__restrict__ rad_id, const double *__restrict__ rad_q, int tile_rads,
                  int n_orb, const double *__restrict__ dia, const double *__restrict__ sx,
                  const double *__restrict__ sy, const double *__restrict__ scale,
-                 long long n_frames, long long frames_per_cta, double *__restrict__ out,
-                 double *__restrict__ gfre, double *__restrict__ gfim, double *__restrict__ gdia,
+                 long long n_frames, long long frames_per_cta, bool zero_dia,
+                 double *__restrict__ out, double *__restrict__ gfre,
+                 double *__restrict__ gfim, double *__restrict__ gdia,
                  double *__restrict__ gsx, double *__restrict__ gsy,
                  double *__restrict__ gscale) {
     using CT2 = typename Pair<CT>::type;
@@ -150,12 +151,15 @@ k_nll_dense_grid(const double *__restrict__ fre, const double *__restrict__ fim,
         for (int i = tid; i < nf * n_rad; i += DG_THREADS) {
             const int f = i / n_rad, j = i - f * n_rad;
             const double pq = DG_PI * rad_q[r0 + j];
-            const CT x = (CT)(pq * dia[d0 + f]);
+            CT x = (CT)(pq * dia[d0 + f]);
+            // a frame without a sphere, as the slices take it (kernels.cu:66-67)
+            const bool zero = zero_dia && x == (CT)0;
+            if (zero) x = (CT)1.e-5;
             CT sn, cs;
             dg_sincos(x, &sn, &cs);
             const CT ix = (CT)1 / x;
             const CT ff = (sn - x * cs) * ix * ix * ix;
-            const CT dff = sn * ix * ix - (CT)3 * ff * ix;
+            const CT dff = zero ? (CT)0 : sn * ix * ix - (CT)3 * ff * ix;
             rt[f * rstride + j] = CT2{ff, dff * (CT)pq};
         }
         __syncthreads();
@@ -269,11 +273,12 @@ bool grid_tables_ok(int precision, long long size, long long n_pix, const int *o
 }
 
 // out += sum_d v s_d (sum_pixels |F + r_d|^2 + bg_sum); F's parts lie fstride
-// doubles apart.
+// doubles apart.  zero_dia: the form factor of diameter 0 is the slices'
+// (without: NaN, as the MaxLP pixels' reference amplitude gives).
 template <typename CT, bool GRAD>
 int launch_dense_grid(const GridTables &g, long long n_pix, int size, const double *fre,
-                      const double *fim, int fstride, double v, double bg_sum, const double *dia,
-                      const double *sx, const double *sy, const double *scale,
+                      const double *fim, int fstride, double v, double bg_sum, bool zero_dia,
+                      const double *dia, const double *sx, const double *sy, const double *scale,
                       long long n_frames, double *out, double *gfre, double *gfim, double *gdia,
                       double *gsx, double *gsy, double *gscale, cudaStream_t stream) {
     if (n_pix == 0) return RSPI_OK;
@@ -293,7 +298,7 @@ int launch_dense_grid(const GridTables &g, long long n_pix, int size, const doub
     k_nll_dense_grid<CT, GRAD><<<grid, DG_THREADS, smem, stream>>>(
         fre, fim, fstride, v, bg_sum, size, reinterpret_cast<const int4 *>(g.order), g.xy, g.rad_id, g.rad_q,
         g.tile_rads, (int)n_orb, dia, sx, sy,
-        scale, n_frames, per, out, gfre, gfim, gdia, gsx, gsy, gscale);
+        scale, n_frames, per, zero_dia, out, gfre, gfim, gdia, gsx, gsy, gscale);
     return RSPI_OK;
 }
 
