@@ -194,13 +194,16 @@ k_nll_dense_grid(const double *__restrict__ fre, const double *__restrict__ fim,
                         gi[k][2] = fma(s2, (double)w2, gi[k][2]);
                         gr[k][3] = fma(s2, (double)z3, gr[k][3]);
                         gi[k][3] = fma(s2, (double)w3, gi[k][3]);
-                        // an opposite pair's terms together: z . e and z . (i r)
-                        const CT ap = z0 + z2, bp = w0 - w2, aq = z1 + z3, bq = w1 - w3;
-                        d64 = fma((double)a.y, (double)(ap * e0 + bp * e1) +
-                                                   (double)(aq * h0 + bq * h1), d64);
-                        const CT cp = bp * er - ap * ei, cq = bq * hr - aq * hi;
-                        x64 += (double)((CT)x * cp - (CT)y * cq);
-                        y64 += (double)((CT)y * cp + (CT)x * cq);
+                        // z . e and z . (i e), the pixels widened before they meet
+                        const double ap = (double)z0 + (double)z2, bp = (double)w0 - (double)w2;
+                        const double aq = (double)z1 + (double)z3, bq = (double)w1 - (double)w3;
+                        const double p0 = (double)e0, p1 = (double)e1;
+                        const double q0 = (double)h0, q1 = (double)h1;
+                        d64 = fma((double)a.y, fma(ap, p0, bp * p1) + fma(aq, q0, bq * q1), d64);
+                        const double ff = (double)a.x;
+                        const double cp = ff * fma(bp, p0, -ap * p1), cq = ff * fma(bq, q0, -aq * q1);
+                        x64 = fma((double)x, cp, fma(-(double)y, cq, x64));
+                        y64 = fma((double)y, cp, fma((double)x, cq, y64));
                     }
                 }
             }
