@@ -180,29 +180,35 @@ static inline int rspi_sm_count() {
     return c;
 }
 
-// Dynamic shared-memory opt-in of one kernel, applied on each device the
-// first time a launch there needs more than the default: one static
-// RspiSmemOptIn per kernel instance.  Concurrent first calls on one device
-// both apply the same attribute, which is harmless.  Returns false when the
-// attribute cannot be set.
+// Dynamic shared-memory opt-in of one kernel: one static RspiSmemOptIn per
+// kernel instance.  The first launch on a device sets the most that the
+// device gives a block beside the kernel's static shared memory, whatever it
+// needs itself: callers with different sizes on several threads then all set
+// the same value, in any order.  Returns false when the attribute cannot be
+// set or `smem` is beyond it.
 struct RspiSmemOptIn {
-    std::atomic<size_t> done[RSPI_MAX_DEVICES];
+    std::atomic<size_t> limit[RSPI_MAX_DEVICES];   // 0: not set yet
 };
 
 static inline bool rspi_smem_optin(const void *kernel, size_t smem, RspiSmemOptIn &st) {
     const int dev = rspi_device();
     const bool cached = dev >= 0 && dev < RSPI_MAX_DEVICES;
-    if (cached && st.done[dev].load(std::memory_order_acquire) >= smem) return true;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
-        return false;
-    if (cached) {
-        size_t prev = st.done[dev].load(std::memory_order_relaxed);
-        while (prev < smem &&
-               !st.done[dev].compare_exchange_weak(prev, smem, std::memory_order_release))
-            ;
+    size_t limit = cached ? st.limit[dev].load(std::memory_order_acquire) : 0;
+    if (limit == 0) {
+        int most = 0;
+        cudaFuncAttributes attr;
+        if (cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) !=
+                cudaSuccess ||
+            cudaFuncGetAttributes(&attr, kernel) != cudaSuccess ||
+            (size_t)most <= attr.sharedSizeBytes)
+            return false;
+        limit = (size_t)most - attr.sharedSizeBytes;
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)limit) != cudaSuccess)
+            return false;
+        if (cached) st.limit[dev].store(limit, std::memory_order_release);
     }
-    return true;
+    return smem <= limit;
 }
 
 static inline unsigned rspi_blocks(long long work, int threads, int cap_per_sm = 8) {
