@@ -183,9 +183,13 @@ k_nll_dense_grid(const double *__restrict__ fre, const double *__restrict__ fim,
                     const CT z1 = f_r[k][1] + hr, w1 = f_i[k][1] + hi;
                     const CT z2 = f_r[k][2] + er, w2 = f_i[k][2] - ei;
                     const CT z3 = f_r[k][3] + hr, w3 = f_i[k][3] - hi;
-                    a64 += ((double)(z0 * z0 + w0 * w0) + (double)(z1 * z1 + w1 * w1)) +
-                           ((double)(z2 * z2 + w2 * w2) + (double)(z3 * z3 + w3 * w3));
-                    if (GRAD) {
+                    if (!GRAD) {
+                        a64 += ((double)(z0 * z0 + w0 * w0) + (double)(z1 * z1 + w1 * w1)) +
+                               ((double)(z2 * z2 + w2 * w2) + (double)(z3 * z3 + w3 * w3));
+                    } else {
+                        // the values are widened for the gradients anyway
+                        auto sq = [](double r, double i, double t) { return fma(r, r, fma(i, i, t)); };
+                        a64 = sq(z0, w0, sq(z1, w1, sq(z2, w2, sq(z3, w3, a64))));
                         gr[k][0] = fma(s2, (double)z0, gr[k][0]);
                         gi[k][0] = fma(s2, (double)w0, gi[k][0]);
                         gr[k][1] = fma(s2, (double)z1, gr[k][1]);
