@@ -34,6 +34,18 @@ SETS_COUNTED_COLS = (1 << 14) - 8   # most columns of a part with counted entrie
 # of 173 likelihood photons, 8.4% fewer entries, 15.9 ms for 16.3 (single
 # entries); of 104, 5.5% fewer, 11.1 for 11.0; of 52, 3% fewer, 7.2 for 7.0.
 COUNT_GAIN = 14
+ROW_SHARED = 220 * 1024          # longest FP64 row that the entries' rescoring keeps on the SM
+# The dense form rescores a candidate over the stored counts of all likelihood
+# columns (rspi_rescore_dense) where the frames' entries fill this part of the
+# columns or more, else over the entries (rspi_rescore): a third where a row
+# exceeds the entries' shared-memory row, two thirds where it fits.  Both, us,
+# entries / columns, at a later and at a first iteration: 600 frames of 255^2
+# (global rows), 6% of the columns 7,700 / 56,000 and 2,700 / 6,500, 37% 8,600 /
+# 8,400 and 6,300 / 5,100, 83% 6,000 / 3,100 and 11,500 / 4,700; 600 of 185^2 7%
+# 2,100 / 28,000 and 940 / 3,500, 61% 2,000 / 2,000 and 1,700 / 2,400, 84%
+# 1,800 / 1,250 and 2,800 / 3,400, 98% 1,200 / 1,040 and 1,900 / 1,070.
+COLUMNS_GLOBAL = 1. / 3.
+COLUMNS_SHARED = 2. / 3.
 SPLIT_SETS = 64                  # sets the frame-set kernel may cut (its limit)
 SPLIT_WARPS = 32                 # warps sharing a tile (the widest CTA)
 # A set longer than three warps' shares of its part is cut into pieces of a
@@ -460,7 +472,12 @@ class EStep:
         self.cand_off = torch.empty(n + 1, dtype=_i64, device=dev)
         self.row_cnt = torch.empty(self.n_rows, dtype=_i32, device=dev)
         self.row_cand_off = torch.empty(self.n_rows + 1, dtype=_i64, device=dev)
-        self._alloc_row_scratch()
+        filled = 32. * self.ll['total_rows'] / max(1, n * self.n_sel)
+        self.rescore_columns = filled >= (COLUMNS_GLOBAL if self.p_pad * 8 > ROW_SHARED
+                                          else COLUMNS_SHARED)
+        self.row_scratch, self.scratch_rows = None, 0
+        if not self.rescore_columns:
+            self._alloc_row_scratch()
         # Error bound of the GEMM value.  The candidate threshold's eps_d is
         # 2^-24 ((rows + 8) photons lmax + |max| + delta + 1) (+ 1e-9 photons
         # lmax).  i8: the quantisation bound 2^-22 photons is rows = 0 with
@@ -711,7 +728,7 @@ class EStep:
         """Global rows for FP64 rescoring when a row exceeds shared memory
         (one per SM; none otherwise)."""
         self.row_scratch, self.scratch_rows = None, 0
-        if self.p_pad * 8 > 220 * 1024:
+        if self.p_pad * 8 > ROW_SHARED:
             sms = torch.cuda.get_device_properties(self.device).multi_processor_count
             self.scratch_rows = int(sms)
             self.row_scratch = torch.empty((sms, self.p_pad), dtype=_f64, device=self.device)
@@ -896,7 +913,7 @@ class EStep:
                     continue
                 self.n_candidates = total
             break
-        if self.form == 'dense':
+        if self.form == 'dense' and self.rescore_columns:
             call('rspi_rescore_dense', ptr(self.cand_d), ptr(self.cand_r), ptr(self.cand_off), n,
                  self.capacity, self.n_rows, ptr(self.ph.frames), ptr(self.holo), self.num_rot,
                  ptr(self.rot_cs), self.size, ptr(self.bg), ptr(self.sel_pix), self.n_sel,
