@@ -430,17 +430,22 @@ __global__ void k_dense_frames_u8(const unsigned short *__restrict__ frames, lon
 // rint(L 2^21) as four 8-bit digit planes b[part][row][c] (zero beyond n_sel).
 // |L| is below 1024 for every value rot_log_value returns (the -1000 sentinel,
 // and logs of doubles); a larger value is clamped and flagged.
-// A CTA takes one rotation j and up to RQ_STATES consecutive states, a warp
-// 128 columns, 32 neighbours at a time: the columns' rotated positions depend
-// on (j, column) only and are computed once for the states, and the four
-// digits of four lanes' columns change places (two shuffles) for one 32-bit
-// store per digit plane.  PAIRS: holo as (w[p], w[p + 1]) pairs, so that a
+// A CTA takes one rotation j, up to RQ_STATES consecutive states and a part of
+// the columns (1,024 or more, for up to RQ_CTAS CTAs per SM: few rows fill the
+// GPU too), a warp 128 columns, 32 neighbours at a time: the columns' rotated
+// positions depend on (j, column) only and are computed once for the states,
+// and the four digits of four lanes' columns change places (two shuffles) for
+// one 32-bit store per digit plane.  PAIRS: holo as (w[p], w[p + 1]) pairs, so that a
 // corner row is one 16-byte load.  Bound by L1 (75% of its wavefronts with
 // four columns of a thread side by side and 8-byte loads) and by issue; 9,720
 // rows x 47,616 columns: 3.25 ms with a row per CTA, 2.99 with eight states,
 // 2.87 with neighbouring columns, 2.67 with pairs and four CTAs per SM (three
-// 2.85, five 2.92; four states 2.81, sixteen 2.99).
+// 2.85, five 2.92; four states 2.81, sixteen 2.99), 2.50 in parts (RQ_CTAS 16
+// 2.66, 32 2.52, 128 2.53).  108 rows of 4 rotations: 0.14 ms with a row per
+// CTA, 0.72 with eight states and all columns, 0.06 in parts; 1,620 rows of
+// 60: 0.63, 0.87, 0.45.
 constexpr int RQ_STATES = 8;
+constexpr int RQ_CTAS = 64;   // per SM
 
 template <bool PAIRS>
 __global__ void __launch_bounds__(256, 4)
@@ -460,7 +465,8 @@ k_rot_log_q(const double *__restrict__ holo, int num_rot, const double *__restri
     while (se > sb && (se - 1) * num_rot + j >= row_end) --se;
     if (sb == se) return;
     const int lane = threadIdx.x & 31, i4 = lane & 3;
-    for (int cb = 4 * (threadIdx.x - lane); cb < k_pad; cb += 4 * blockDim.x) {
+    for (int cb = 4 * (blockIdx.y * blockDim.x + threadIdx.x - lane); cb < k_pad;
+         cb += 4 * blockDim.x * gridDim.y) {
         const int c0 = cb + lane;  // columns c0 + 32 u (k_pad is a multiple of 128)
         int at[4];                 // first corner; -1: outside the detector, -2: no column
         double fx[4], fy[4], bgv[4];
@@ -672,7 +678,10 @@ static int rot_log_fixed(const double *holo, long long n_states0, long long num_
     const long long blocks = ((s_hi - s_lo) / RQ_STATES + 1) * num_rot;
     if (blocks > 0x7fffffffLL || k_pad > 0x7fffffffLL || num_rot > 0x7fffffffLL)
         return RSPI_ERR_ARG;
-    k_rot_log_q<PAIRS><<<(unsigned)blocks, 256, 0, stream>>>(
+    // a part of the columns per CTA, of a thread's four at least
+    const long long parts = min((k_pad + 1023) / 1024,
+                                max(1LL, (long long)RQ_CTAS * rspi_sm_count() / blocks));
+    k_rot_log_q<PAIRS><<<dim3((unsigned)blocks, (unsigned)parts), 256, 0, stream>>>(
         holo, (int)num_rot, rot_cs, (int)size, bg, sel_pix, (int)n_sel, (int)k_pad, row_begin,
         row_end, s_lo, plane_rows * k_pad, (uint8_t *)digits, err);
     RSPI_RETURN_LAUNCH();
