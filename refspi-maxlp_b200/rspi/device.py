@@ -661,16 +661,20 @@ class EStep:
             ps = torch.empty(self.lib.rspi_sets_part_sums_floats(n_sets, ps_ctas),
                              dtype=torch.float32, device=dev)
         items, item_off, slots = self._sets_items(groups, qgroups, goff, parts, n_sets)
-        seg_ctas = self.n_ctas if self.n_ctas > 0 else \
-            torch.cuda.get_device_properties(dev).multi_processor_count
-        seg = torch.empty(seg_ctas * slots * 128, dtype=torch.float32, device=dev) \
-            if slots else None
+        seg_ctas = max(self.n_ctas,
+                       torch.cuda.get_device_properties(dev).multi_processor_count)
+        seg = self._seg_sums(slots, seg_ctas)
         return dict(entries=entries, group_off=goff, quarter_groups=qgroups,
                     total_groups=total, tile=4, sets=True, counted=counted, items=items,
                     item_off=item_off, seg_sums=seg, seg_slots=slots, seg_ctas=seg_ctas,
                     set_frames=set_frames, col_of_frame=col_of_frame, n_sets=n_sets,
                     frame_groups=frame_groups, n_parts=parts, part_w=part_w, part_sums=ps,
                     part_sums_ctas=ps_ctas, counts=counts)
+
+    def _seg_sums(self, slots, ctas):
+        """Sums of the cut sets' pieces, ``slots`` of 32 x 4 per CTA."""
+        return torch.empty(ctas * slots * 128, dtype=torch.float32, device=self.device) \
+            if slots else None
 
     @staticmethod
     def _sets_items(groups, qgroups, goff, parts, n_sets):
@@ -835,11 +839,14 @@ class EStep:
                  self.n_ctas, cur_stream())
         elif self.kernel == 'sets':
             w = self.wide
-            if self.n_ctas > 0 and self.n_ctas != w['seg_ctas']:
+            if w['n_parts'] > 1 and self.n_ctas > 0 and self.n_ctas != w['part_sums_ctas']:
                 w = self.wide = self._sets_entries()
+            if w['seg_slots'] and self.n_ctas > w['seg_ctas']:
+                w.update(seg_ctas=self.n_ctas, seg_sums=self._seg_sums(w['seg_slots'], self.n_ctas))
             call('rspi_screen_loglike_items', ptr(lsl), self.num_rot, ptr(self.init),
                  ptr(self.ph.scales), ptr(w['entries']), int(w['counted']), ptr(w['group_off']),
-                 ptr(w['quarter_groups']), ptr(w['items']), ptr(w['item_off']), ptr(w['seg_sums']), w['seg_slots'], w['seg_ctas'],
+                 ptr(w['quarter_groups']), ptr(w['items']), ptr(w['item_off']),
+                 ptr(w['seg_sums']), w['seg_slots'], w['seg_ctas'],
                  ptr(w['set_frames']), w['n_sets'], w['n_parts'], w['part_w'], r0, r1,
                  ptr(self.prob[r0]), self.n_cols, ptr(w['part_sums']), w['part_sums_ctas'],
                  ptr(self.frame_max), self.warps, self.n_ctas, ptr(self.ph.err.t), cur_stream())
