@@ -53,6 +53,7 @@ SPLIT_WARPS = 32                 # warps sharing a tile (the widest CTA)
 # larger headers cost more: 1,000 frames, longest set 2.3 shares, 0.68 ms
 # whole and 0.70 cut; 4,001 frames, longest 9 shares, 7.45 whole and 6.68 cut.
 SPLIT_SHARES = 3
+MERGE_IMAGES = 1 << 30           # bytes of the merge's images (2 per SM up to 670^2 pixels)
 PIXEL_MAP_MAX_ROT = 1024         # rotation tables the M-step's pixel map serves
 PIXEL_MAP_MAX = 1 << 26          # (rotation, detector pixel) entries of that map
 
@@ -969,9 +970,11 @@ class Merge:
         self.intens = torch.empty((n0, npix), dtype=_f64, device=dev)
         n = estep.ph.num_data
         if estep.form != 'fp64':
-            # an unrotated image per CTA of the row-grouped scatter, two per SM
+            # an unrotated image per CTA of the row-grouped scatter: two per SM,
+            # no more than rows, and within MERGE_IMAGES bytes
             sms = torch.cuda.get_device_properties(dev).multi_processor_count
-            self.images = torch.empty((2 * sms, npix), dtype=_f64, device=dev)
+            n_images = max(1, min(2 * sms, estep.n_rows, MERGE_IMAGES // (8 * npix)))
+            self.images = torch.empty((n_images, npix), dtype=_f64, device=dev)
             self.row_done = torch.empty(estep.n_rows, dtype=_i32, device=dev)
         else:
             self.cnt_part = torch.empty(n * 32, dtype=_i32, device=dev)
