@@ -53,6 +53,9 @@ SPLIT_WARPS = 32                 # warps sharing a tile (the widest CTA)
 # larger headers cost more: 1,000 frames, longest set 2.3 shares, 0.68 ms
 # whole and 0.70 cut; 4,001 frames, longest 9 shares, 7.45 whole and 6.68 cut.
 SPLIT_SHARES = 3
+# Bytes of the dense form's paired slices, twice the slices' own; beyond, its
+# digits come from the plain ones (9,720 rows of 47,616 columns: 2.87 ms for 2.67).
+DENSE_PAIRS = 8 << 30
 MERGE_IMAGES = 1 << 30           # bytes of the merge's images (2 per SM up to 670^2 pixels)
 PIXEL_MAP_MAX_ROT = 1024         # rotation tables the M-step's pixel map serves
 PIXEL_MAP_MAX = 1 << 26          # (rotation, detector pixel) entries of that map
@@ -451,8 +454,10 @@ class EStep:
         self.msum = torch.empty(self.n_states0, dtype=_f64, device=dev)
         self.vscale = torch.empty(1, dtype=_f64, device=dev)
         self.init = torch.empty(self.n_states0, dtype=_f64, device=dev)
+        self.holo_pairs = None
         if gemm == 'i8':
-            self.holo_pairs = torch.empty((self.n_states0, npix, 2), dtype=_f64, device=dev)
+            if self.n_states0 * npix * 16 <= DENSE_PAIRS:
+                self.holo_pairs = torch.empty((self.n_states0, npix, 2), dtype=_f64, device=dev)
             self.lsl = torch.empty((4, self.chunk_rows, self.k_pad), dtype=torch.uint8, device=dev)
         else:
             self.lsl_hi = torch.empty((self.chunk_rows, self.k_pad), dtype=torch.bfloat16,
@@ -763,7 +768,7 @@ class EStep:
                  self.n_sel, ptr(self.holo[g0]), ptr(self.msum[g0:]), s)
         call('rspi_vscale_init', ptr(self.msum), self.n_states0, ptr(self.ph.powder),
              ptr(self.sel_pix), self.n_sel, ptr(self.vscale), ptr(self.init), s)
-        if self.form != 'dense' or self.dense_gemm == 'i8':
+        if self.holo_pairs is not None:
             call('rspi_holo_pairs', ptr(self.holo), self.n_states0, self.size,
                  ptr(self.holo_pairs), s)
         if self.form != 'fp64':
@@ -779,7 +784,9 @@ class EStep:
     def rot_slices(self, r0, r1, out=None):
         """a6: rotated log-slices of rows [r0, r1) into ``out`` (or the chunk buffer)."""
         if self.form == 'dense' and self.dense_gemm == 'i8':
-            call('rspi_rot_log_fixed_pairs', ptr(self.holo_pairs), self.n_states0, self.num_rot,
+            name, holo = ('rspi_rot_log_fixed', self.holo) if self.holo_pairs is None else \
+                ('rspi_rot_log_fixed_pairs', self.holo_pairs)
+            call(name, ptr(holo), self.n_states0, self.num_rot,
                  ptr(self.rot_cs), self.size, ptr(self.bg), ptr(self.sel_pix), self.n_sel,
                  self.k_pad, r0, r1, self.chunk_rows, ptr(self.lsl), ptr(self.ph.err.t),
                  cur_stream())
