@@ -80,6 +80,8 @@ int rspi_ll_entry_rows(const int *ones, const int *multi, const long long *ones_
                        cudaStream_t stream);
 int rspi_scan_rows(const int *frame_rows, long long n_data, long long *row_off,
                    cudaStream_t stream);
+/* Kernels that a scan of n counts launches (1 or 3). */
+int rspi_scan_launches(long long n);
 int rspi_ll_entry_fill(const int *ones, const int *multi, const long long *ones_accum,
                        const long long *multi_accum, const int *place_ones,
                        const int *place_multi, const int *count_multi,

@@ -133,6 +133,10 @@ int rspi_scan_i32(const int *cnt, long long n, long long *off, cudaStream_t stre
     RSPI_RETURN_LAUNCH();
 }
 
+extern "C" int rspi_scan_launches(long long n) {
+    return (n + SCAN_TILE - 1) / SCAN_TILE <= SCAN_ONE ? 1 : 3;
+}
+
 extern "C" int rspi_scan_rows(const int *frame_rows, long long n_data, long long *row_off,
                               cudaStream_t stream) {
     if (n_data <= 0 || !frame_rows || !row_off) return RSPI_ERR_ARG;

@@ -21,6 +21,7 @@ SIGNATURES = {
     'rspi_photon_offsets': (I, [P, P, P, L, P, P, P, P, P, P, I, P, P]),
     'rspi_powder': (I, [P, L, P, P, L, L, L, P, P, P]),
     'rspi_ll_entry_rows': (I, [P, P, P, P, P, P, P, P, L, L, P, P, P, P]),
+    'rspi_scan_launches': (I, [L]),
     'rspi_scan_rows': (I, [P, L, P, P]),
     'rspi_ll_entry_fill': (I, [P, P, P, P, P, P, P, P, L, L, P, P, P, P]),
     'rspi_holo_slices': (I, [P, P, P, P, L, L, P, P, L, P, P, P]),
@@ -167,6 +168,15 @@ KERNELS_PER_CALL = {
     'rspi_dense_loglike_i8': 1, 'rspi_sets_entries_check': 1, 'rspi_sim_views': 1, 'rspi_sim_counts': 1,
     'rspi_sim_poisson': 1, 'rspi_sim_sparse_counts': 1, 'rspi_sim_sparse_fill': 1,
 }
+# counts scanned by an entry point, from its arguments; its scan's launches
+# beyond the one in KERNELS_PER_CALL follow from them (rspi_scan_launches)
+SCANNED = {
+    'rspi_scan_rows': lambda a: a[1], 'rspi_screen_candidates': lambda a: a[2],
+    'rspi_screen_candidates_cols': lambda a: a[4],
+    'rspi_screen_candidates_noalloc': lambda a: a[2], 'rspi_rescore': lambda a: a[5],
+    'rspi_rescore_cols': lambda a: a[5], 'rspi_rescore_dense': lambda a: a[5],
+    'rspi_posterior_pairs': lambda a: a[2], 'rspi_maxlp_pixel_map': lambda a: a[1] * a[2] ** 2,
+}
 launch_count = 0
 
 
@@ -175,3 +185,5 @@ def call(name, *args):
     global launch_count
     check(getattr(load(), name)(*args), name)
     launch_count += KERNELS_PER_CALL.get(name, 0)
+    if name in SCANNED:
+        launch_count += load().rspi_scan_launches(SCANNED[name](args)) - 1
