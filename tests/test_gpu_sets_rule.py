@@ -1,0 +1,32 @@
+"""The layouts that the shipped rules choose: a set far longer than a warp's
+share is cut, one that is not stays whole; entries of several photons where
+they leave out one entry in COUNT_GAIN or more, single ones elsewhere."""
+import numpy as np
+import pytest
+
+from oracle import emc_oracle as E
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize('heavy,mean,cut,counted', [
+    (40000, 0.02, True, True),       # one frame of many photons per pixel among light ones
+    (0, 0.02, False, False),         # 1,300 alike frames, pixels seldom repeat
+    (0, 1.5, False, True)])          # 1,300 alike, most pixels repeat
+def test_shipped_rules(heavy, mean, cut, counted):
+    from rspi.photonfile import sparse_from_dense
+    from test_gpu_estep import _estep, _photons
+    size, n = 31, 1300               # 41 sets for 32 warps
+    rng = np.random.default_rng(4)
+    frames = rng.poisson(mean, (n, size * size))
+    if heavy:
+        frames[7] = rng.poisson(heavy / size ** 2, size * size)
+    d = sparse_from_dense(frames)
+    ds = E.parse_photons(d['ones'], d['multi'], d['place_ones'], d['place_multi'],
+                         d['count_multi'], size * size, True)
+    sx, sy, dia, _ = E.generate_states((0., 1., 2), (0., 0., 1), (6., 8., 2))
+    es = _estep(_photons(ds, False), size, 3, sx, sy, dia, ds['bg'], form='screen',
+                states_per_tile=4)
+    assert es.kernel == 'sets'
+    assert (es.wide['seg_slots'] > 0) == cut
+    assert es.wide['counted'] == counted
