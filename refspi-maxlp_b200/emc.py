@@ -129,7 +129,8 @@ class EMC():
                            slice_budget_bytes=int(self.slice_budget_gb * (1 << 30)),
                            n_modes=self.num_modes, dense_gemm=self.dense_gemm,
                            dense_rescore=self.dense_rescore, kernel=self.kernel,
-                           slice_math=self.slice_math, set_order=self.set_order)
+                           slice_math=self.slice_math, set_order=self.set_order,
+                           entries='auto')
         self.merger = None
         self.intens = None
         if self.merge_intens:

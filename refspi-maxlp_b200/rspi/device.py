@@ -275,18 +275,24 @@ class EStep:
     (frame-set kernel): ``grouped`` (default) picks each quarter warp's
     eight frames among 256 of alike photon count so that their bank-class
     totals stay close to their mean (``rspi_sets_group``); ``rank`` takes
-    them in rank order.
+    them in rank order.  ``entries`` (frame-set kernel): ``auto`` (the default
+    kernel's) gives a pixel of several photons one entry per binary digit
+    where that leaves out enough of them; ``single``, the layout when
+    ``kernel`` alone names it, an entry per photon.
     """
 
     def __init__(self, photons, size, num_rot, shiftx, shifty, sphere_dia, probmask, bg,
                  form='fp64', states_per_tile=None, warps=32, n_ctas=0,
                  slice_budget_bytes=8 << 30, delta=20., cand_per_frame=None, kernel=None,
                  n_modes=1, dense_gemm='auto', dense_rescore=True, screen_parts=None,
-                 slice_math=None, set_order='grouped'):
+                 slice_math=None, set_order='grouped', entries=None):
         if form not in ('fp64', 'screen', 'dense'):
             raise ValueError('form must be fp64, screen or dense')
-        # entries of several photons: only where the layout is left to choose
-        self.count_entries = kernel is None
+        if entries is None:
+            entries = 'auto' if kernel is None else 'single'
+        if entries not in ('auto', 'single'):
+            raise ValueError('entries must be auto or single')
+        self.count_entries = entries == 'auto'
         if kernel is None:   # default likelihood kernel of each form
             kernel = 'sets' if form == 'screen' else 'stream'
         kernels = {'fp64': ('stream', 'dynamic'), 'screen': ('stream', 'quad4', 'sets'),

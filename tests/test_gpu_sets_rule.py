@@ -30,3 +30,18 @@ def test_shipped_rules(heavy, mean, cut, counted):
     assert es.kernel == 'sets'
     assert (es.wide['seg_slots'] > 0) == cut
     assert es.wide['counted'] == counted
+
+
+@pytest.mark.parametrize('extra', ['', 'kernel = sets\n'])
+def test_a_configuration_that_names_the_kernel_keeps_its_layout(extra, tmp_path):
+    """`kernel = sets` asks for what is the default anyway: the same entries."""
+    from emc import EMC
+    from helpers import write_case
+    from rspi.photonfile import sparse_from_dense
+    size = 31
+    rng = np.random.default_rng(5)
+    data = dict(sparse_from_dense(rng.poisson(1.5, (40, size * size))),
+                num_pix=np.array([size * size]))
+    rec = EMC(write_case(str(tmp_path), data=data, size=size, num_rot=3, shiftx='0 1 2',
+                         shifty='0 0 1', sphere_dia='6 8 2', need_scaling=True, extra=extra))
+    assert rec.estep.kernel == 'sets' and rec.estep.wide['counted']
