@@ -24,6 +24,7 @@ with CUDA events and extrapolate linearly to a whole iteration.
 """
 import ctypes
 import os
+import unittest
 
 import numpy as np
 import torch
@@ -36,12 +37,17 @@ _P, _L, _I, _U, _D = (ctypes.c_void_p, ctypes.c_longlong, ctypes.c_int, ctypes.c
 _lib = None
 
 
+class NotBuilt(FileNotFoundError, unittest.SkipTest):
+    """The reference's source tree was not there to build its kernels from: a
+    test that compares with them is skipped."""
+
+
 def load():
-    """The reference kernels for the GPU; raises if they were not built."""
+    """The reference kernels for the GPU; raises NotBuilt if there are none."""
     global _lib
     if _lib is None:
         if not os.path.exists(LIB):
-            raise FileNotFoundError('%s is not built (oracle/ref_gpu/build.py)' % LIB)
+            raise NotBuilt('%s is not built (oracle/ref_gpu/build.py)' % LIB)
         lib = ctypes.CDLL(LIB)
         lib.ref_gpu_slice_gen.argtypes = [_U, _U, _U, _U, _P, _D, _D, _L, _P, _L, _P, _P]
         lib.ref_gpu_slice_gen_holo.argtypes = [_U, _U, _U, _U, _P, _D, _D, _D, _D, _D, _L, _P,
