@@ -167,8 +167,8 @@ def start_model(cfg_id, w):
 
 def dram_traffic(args, w, es, rows_per_launch):
     """DRAM bytes (read + write) of one likelihood launch from the committed
-    ncu capture of the same workload (form, configuration, frames, rows per
-    launch), or None when no capture matches."""
+    ncu capture of the same workload (form, kernel and its entries' layout,
+    configuration, frames, rows per launch), or None when no capture matches."""
     path = os.path.join(REPO, 'profiles', 'k_screen_config2_dram.json')
     try:
         with open(path) as f:
@@ -176,8 +176,12 @@ def dram_traffic(args, w, es, rows_per_launch):
     except (OSError, ValueError, KeyError):
         return None
     kern = es.kernel
+    wide = es.wide or {}
+    layout = ('counted' if wide.get('counted') else 'single') + \
+        ('-cut' if wide.get('seg_slots') else '')
     for c in caps:
         if (c['form'] == es.form and c.get('kernel', 'stream') == kern and
+                c.get('entries', 'single') == layout and
                 c['config'] == args.config and c['frames'] == w['n'] and
                 c['rows_per_launch'] == int(round(rows_per_launch))):
             return float(c['dram_bytes_read'] + c['dram_bytes_write'])
@@ -220,6 +224,8 @@ def roofline_blocks(args, w, es, ll_ms, ll_launches, ms, clk, pk, sm_count):
     # algorithmic bytes per launch = its slices in + its LL rows out + the
     # packed photon entries once
     ent_bytes = total_rows * 32 * (2 if es.form == 'screen' else 4)
+    if es.wide is not None and es.wide.get('counted'):
+        ent_bytes = 2 * int(es.wide['counts'].sum().item())   # entries of several photons
     alg_bytes = rows_per_launch * (es.p_row * esz + w['n'] * osz) + ent_bytes + 8 * w['n']
     achieved = alg_bytes / (ll_launch_ms * 1e-3) / 1e9
     # on-chip gather roofline.  Screened form: one shared-memory value per

@@ -801,14 +801,15 @@ int rspi_nll(int precision, int want_grad, const int *ones, const int *multi,
  * (last - first + 1) of a group's rad_id.  order on a 16-byte boundary.
  * Sizes whose tables exceed shared memory: RSPI_ERR_ARG. */
 int rspi_nll_grid(int precision, int want_grad, const int *ones, const int *multi,
-             const long long *ones_accum, const long long *multi_accum, const int *place_ones,
-             const int *place_multi, const int *count_multi, long long n_frames,
-             const double *rot_cs, long long size, const int *mask_idx, long long n_pix, const int *order,
-                  const int *xy, const int *rad_id, const double *rad_q, int tile_rads,
-             const double *fre, const double *fim, const double *qx, const double *qy,
-             const double *qrad, const double *dia, const double *sx, const double *sy,
-             const double *scale, double *nll, double *gfre, double *gfim, double *gdia,
-             double *gsx, double *gsy, double *gscale, int *err, cudaStream_t stream);
+                  const long long *ones_accum, const long long *multi_accum,
+                  const int *place_ones, const int *place_multi, const int *count_multi,
+                  long long n_frames, const double *rot_cs, long long size, const int *mask_idx,
+                  long long n_pix, const int *order, const int *xy, const int *rad_id,
+                  const double *rad_q, int tile_rads, const double *fre, const double *fim,
+                  const double *qx, const double *qy, const double *qrad, const double *dia,
+                  const double *sx, const double *sy, const double *scale, double *nll,
+                  double *gfre, double *gfim, double *gdia, double *gsx, double *gsy,
+                  double *gscale, int *err, cudaStream_t stream);
 
 /* Orbits per group of rspi_nll_grid for a size^2 detector; -1: a detector too
  * large for its tables (rspi_nll takes it), or an unknown precision. */
@@ -842,15 +843,15 @@ int rspi_emc_nll(int precision, int want_grad, const double *model, long long si
  * tables of the likelihood pixels (order holds flat pixel numbers, rad_q the
  * radii over size), and bg_sum their background's sum. */
 int rspi_emc_nll_grid(int precision, int want_grad, const double *model, long long size,
-                 const double *bg, const int *sel_pix, long long n_sel, const int *order,
+                      const double *bg, const int *sel_pix, long long n_sel, const int *order,
                       const int *xy, const int *rad_id, const double *rad_q, int tile_rads,
-                      double bg_sum, const int *pix2sel,
-                 const int *ones, const int *multi, const long long *ones_accum,
-                 const long long *multi_accum, const int *place_ones, const int *place_multi,
-                 const int *count_multi, long long n_frames, const double *rot_cs,
-                 const double *dia, const double *sx, const double *sy, const double *scale,
-                 double vscale, double *nll, double *gre, double *gim, double *gdia,
-                 double *gsx, double *gsy, double *gscale, int *err, cudaStream_t stream);
+                      double bg_sum, const int *pix2sel, const int *ones, const int *multi,
+                      const long long *ones_accum, const long long *multi_accum,
+                      const int *place_ones, const int *place_multi, const int *count_multi,
+                      long long n_frames, const double *rot_cs, const double *dia,
+                      const double *sx, const double *sy, const double *scale, double vscale,
+                      double *nll, double *gre, double *gim, double *gdia, double *gsx,
+                      double *gsy, double *gscale, int *err, cudaStream_t stream);
 
 /* ------------------------------------------------------------ model refinement
  * Error reduction and difference map after the pattern search

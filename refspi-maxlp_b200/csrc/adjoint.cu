@@ -250,13 +250,14 @@ int launch_dense(const GridTables &g, long long n_pix, int size, const double *f
 }
 
 template <typename CT, bool GRAD>
-int launch_all(const GridTables &g, const int *ones, const int *multi, const long long *oacc, const long long *macc,
-                const int *po, const int *pm, const int *cm, long long n_frames,
-                const double *rot_cs, int size, const int *mask_idx, long long n_pix,
-                const double *fre, const double *fim, const double *qx, const double *qy,
-                const double *qrad, const double *dia, const double *sx, const double *sy,
-                const double *scale, double *out, double *gfre, double *gfim, double *gdia,
-                double *gsx, double *gsy, double *gscale, int *err, cudaStream_t stream) {
+int launch_all(const GridTables &g, const int *ones, const int *multi, const long long *oacc,
+               const long long *macc, const int *po, const int *pm, const int *cm,
+               long long n_frames, const double *rot_cs, int size, const int *mask_idx,
+               long long n_pix, const double *fre, const double *fim, const double *qx,
+               const double *qy, const double *qrad, const double *dia, const double *sx,
+               const double *sy, const double *scale, double *out, double *gfre, double *gfim,
+               double *gdia, double *gsx, double *gsy, double *gscale, int *err,
+               cudaStream_t stream) {
     const int st = launch_dense<CT, GRAD>(g, n_pix, size, fre, fim, qx, qy, qrad, dia, sx, sy,
                                           scale, n_frames, out, gfre, gfim, gdia, gsx, gsy,
                                           gscale, stream);
@@ -270,16 +271,16 @@ int launch_all(const GridTables &g, const int *ones, const int *multi, const lon
 
 }  // namespace
 
-static int nll_entry(const GridTables &g, int precision, int want_grad, const int *ones, const int *multi,
-                        const long long *ones_accum, const long long *multi_accum,
-                        const int *place_ones, const int *place_multi, const int *count_multi,
-                        long long n_frames, const double *rot_cs, long long size,
-                        const int *mask_idx, long long n_pix, const double *fre,
-                        const double *fim, const double *qx, const double *qy,
-                        const double *qrad, const double *dia, const double *sx,
-                        const double *sy, const double *scale, double *nll, double *gfre,
-                        double *gfim, double *gdia, double *gsx, double *gsy, double *gscale,
-                        int *err, cudaStream_t stream) {
+static int nll_entry(const GridTables &g, int precision, int want_grad, const int *ones,
+                     const int *multi, const long long *ones_accum,
+                     const long long *multi_accum, const int *place_ones,
+                     const int *place_multi, const int *count_multi, long long n_frames,
+                     const double *rot_cs, long long size, const int *mask_idx,
+                     long long n_pix, const double *fre, const double *fim, const double *qx,
+                     const double *qy, const double *qrad, const double *dia, const double *sx,
+                     const double *sy, const double *scale, double *nll, double *gfre,
+                     double *gfim, double *gdia, double *gsx, double *gsy, double *gscale,
+                     int *err, cudaStream_t stream) {
     if (n_frames <= 0 || n_frames > 0x7fffffffLL * DT_FRAMES || size <= 1 || size > 46340 ||
         n_pix < 0 || !ones || !multi || !ones_accum || !multi_accum || !rot_cs || !mask_idx ||
         !fre || !fim || !qx || !qy || !qrad || !dia || !sx || !sy || !scale || !nll ||
@@ -296,9 +297,10 @@ static int nll_entry(const GridTables &g, int precision, int want_grad, const in
         cudaMemsetAsync(gscale, 0, sizeof(double) * n_frames, stream);
     }
 #define RSPI_NLL(CT, G)                                                                          \
-    launch_all<CT, G>(g, ones, multi, ones_accum, multi_accum, place_ones, place_multi, count_multi, \
-                      n_frames, rot_cs, (int)size, mask_idx, n_pix, fre, fim, qx, qy, qrad, dia,  \
-                      sx, sy, scale, nll, gfre, gfim, gdia, gsx, gsy, gscale, err, stream)
+    launch_all<CT, G>(g, ones, multi, ones_accum, multi_accum, place_ones, place_multi,          \
+                      count_multi, n_frames, rot_cs, (int)size, mask_idx, n_pix, fre, fim, qx,   \
+                      qy, qrad, dia, sx, sy, scale, nll, gfre, gfim, gdia, gsx, gsy, gscale,     \
+                      err, stream)
     if (precision == 1 && want_grad) return RSPI_NLL(double, true);
     if (precision == 1) return RSPI_NLL(double, false);
     if (want_grad) return RSPI_NLL(float, true);

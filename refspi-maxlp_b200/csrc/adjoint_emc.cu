@@ -271,18 +271,19 @@ k_emc_nll_photons(const int *__restrict__ ones, const int *__restrict__ multi,
 }
 
 template <typename CT, bool GRAD>
-int emc_launch(const GridTables &g, double bg_sum, const double2 *model, int size, const double *bg, const int *sel_pix,
-                long long n_sel, const int *pix2sel, const int *ones, const int *multi,
-                const long long *oacc, const long long *macc, const int *po, const int *pm,
-                const int *cm, long long n_frames, const double *rot_cs, const double *dia,
-                const double *sx, const double *sy, const double *scale, double vscale,
-                double *out, double *gre, double *gim, double *gdia, double *gsx, double *gsy,
-                double *gscale, int *err, cudaStream_t stream) {
+int emc_launch(const GridTables &g, double bg_sum, const double2 *model, int size,
+               const double *bg, const int *sel_pix, long long n_sel, const int *pix2sel,
+               const int *ones, const int *multi, const long long *oacc, const long long *macc,
+               const int *po, const int *pm, const int *cm, long long n_frames,
+               const double *rot_cs, const double *dia, const double *sx, const double *sy,
+               const double *scale, double vscale, double *out, double *gre, double *gim,
+               double *gdia, double *gsx, double *gsy, double *gscale, int *err,
+               cudaStream_t stream) {
     if (g.order) {
         const double *m = reinterpret_cast<const double *>(model);
-        const int st = launch_dense_grid<CT, GRAD>(g, n_sel, size, m, m + 1, 2, vscale, bg_sum, true,
-                                                   dia, sx, sy, scale, n_frames, out, gre, gim, gdia,
-                                                   gsx, gsy, gscale, stream);
+        const int st = launch_dense_grid<CT, GRAD>(g, n_sel, size, m, m + 1, 2, vscale, bg_sum,
+                                                   true, dia, sx, sy, scale, n_frames, out, gre,
+                                                   gim, gdia, gsx, gsy, gscale, stream);
         if (st != RSPI_OK) return st;
     } else if (n_sel > 0) {
         const dim3 grid((unsigned)((n_sel + 255) / 256),
@@ -299,16 +300,16 @@ int emc_launch(const GridTables &g, double bg_sum, const double2 *model, int siz
 
 }  // namespace
 
-static int emc_nll_entry(const GridTables &g, double bg_sum, int precision, int want_grad, const double *model, long long size,
-                            const double *bg, const int *sel_pix, long long n_sel,
-                            const int *pix2sel, const int *ones, const int *multi,
-                            const long long *ones_accum, const long long *multi_accum,
-                            const int *place_ones, const int *place_multi,
-                            const int *count_multi, long long n_frames, const double *rot_cs,
-                            const double *dia, const double *sx, const double *sy,
-                            const double *scale, double vscale, double *nll, double *gre,
-                            double *gim, double *gdia, double *gsx, double *gsy, double *gscale,
-                            int *err, cudaStream_t stream) {
+static int emc_nll_entry(const GridTables &g, double bg_sum, int precision, int want_grad,
+                         const double *model, long long size, const double *bg,
+                         const int *sel_pix, long long n_sel, const int *pix2sel,
+                         const int *ones, const int *multi, const long long *ones_accum,
+                         const long long *multi_accum, const int *place_ones,
+                         const int *place_multi, const int *count_multi, long long n_frames,
+                         const double *rot_cs, const double *dia, const double *sx,
+                         const double *sy, const double *scale, double vscale, double *nll,
+                         double *gre, double *gim, double *gdia, double *gsx, double *gsy,
+                         double *gscale, int *err, cudaStream_t stream) {
     if (n_frames <= 0 || n_frames > 0xffffLL * EN_FRAMES || size <= 1 || size > 46340 ||
         n_sel < 0 || (n_sel > 0 && !sel_pix) || !model || !bg || !pix2sel || !ones || !multi ||
         !ones_accum || !multi_accum || !rot_cs || !dia || !sx || !sy || !scale || !nll ||
@@ -326,10 +327,11 @@ static int emc_nll_entry(const GridTables &g, double bg_sum, int precision, int 
         cudaMemsetAsync(gscale, 0, sizeof(double) * n_frames, stream);
     }
     const double2 *m = reinterpret_cast<const double2 *>(model);
-#define RSPI_ENLL(CT, G)                                                                           \
-    emc_launch<CT, G>(g, bg_sum, m, (int)size, bg, sel_pix, n_sel, pix2sel, ones, multi, ones_accum, \
-                      multi_accum, place_ones, place_multi, count_multi, n_frames, rot_cs, dia, \
-                      sx, sy, scale, vscale, nll, gre, gim, gdia, gsx, gsy, gscale, err, stream)
+#define RSPI_ENLL(CT, G)                                                                         \
+    emc_launch<CT, G>(g, bg_sum, m, (int)size, bg, sel_pix, n_sel, pix2sel, ones, multi,         \
+                      ones_accum, multi_accum, place_ones, place_multi, count_multi, n_frames,   \
+                      rot_cs, dia, sx, sy, scale, vscale, nll, gre, gim, gdia, gsx, gsy, gscale, \
+                      err, stream)
     if (precision == 1 && want_grad) return RSPI_ENLL(double, true);
     if (precision == 1) return RSPI_ENLL(double, false);
     if (want_grad) return RSPI_ENLL(float, true);
@@ -355,15 +357,17 @@ extern "C" int rspi_emc_nll(int precision, int want_grad, const double *model, l
                          gre, gim, gdia, gsx, gsy, gscale, err, stream);
 }
 
-extern "C" int rspi_emc_nll_grid(int precision, int want_grad, const double *model, long long size,
-                                 const double *bg, const int *sel_pix, long long n_sel, const int
-                                 *order, const int *xy, const int *rad_id, const double *rad_q, int
-                                 tile_rads, double bg_sum, const int *pix2sel, const int *ones,
-                                 const int *multi, const long long *ones_accum, const long long
-                                 *multi_accum, const int *place_ones, const int *place_multi, const
-                                 int *count_multi, long long n_frames, const double *rot_cs, const
-                                 double *dia, const double *sx, const double *sy, const double
-                                 *scale, double vscale, double *nll, double *gre, double *gim,
+extern "C" int rspi_emc_nll_grid(int precision, int want_grad, const double *model,
+                                 long long size, const double *bg, const int *sel_pix,
+                                 long long n_sel, const int *order, const int *xy,
+                                 const int *rad_id, const double *rad_q, int tile_rads,
+                                 double bg_sum, const int *pix2sel, const int *ones,
+                                 const int *multi, const long long *ones_accum,
+                                 const long long *multi_accum, const int *place_ones,
+                                 const int *place_multi, const int *count_multi,
+                                 long long n_frames, const double *rot_cs, const double *dia,
+                                 const double *sx, const double *sy, const double *scale,
+                                 double vscale, double *nll, double *gre, double *gim,
                                  double *gdia, double *gsx, double *gsy, double *gscale, int *err,
                                  cudaStream_t stream) {
     if (!grid_tables_ok(precision, size, n_sel, order, xy, rad_id, rad_q, tile_rads))

@@ -1187,8 +1187,8 @@ extern "C" int rspi_screen_loglike_items(
         (reinterpret_cast<uintptr_t>(seg_sums) & 15) != 0)
         return RSPI_ERR_ARG;
     return screen_sets_any(lslices_sets, num_rot, init, scales, entries, counted != 0, group_off,
-                           quarter_groups, items, item_off, seg_sums, seg_slots, seg_ctas, set_frames,
-                           n_sets, n_parts, part_w, row_begin, row_end, ll, ll_stride, part_sums,
+                           quarter_groups, items, item_off, seg_sums, seg_slots, seg_ctas,
+                           set_frames, n_sets, n_parts, part_w, row_begin, row_end, ll, ll_stride, part_sums,
                            part_sums_ctas, frame_max, warps_per_cta, n_ctas, err, stream);
 }
 

@@ -608,7 +608,7 @@ k_pattern(double2 *__restrict__ fconv, const int *__restrict__ pixels,
 // ms (2.06), 41^2 with 60 frames 0.30 ms (0.42); 1.3 finalists an iteration
 // instead of 43 at the first.
 constexpr int PS_THREADS = 128;
-constexpr int PS_CTAS = 6;                         // CTAs per SM (80 registers; 5 and 8 measured within 3%)
+constexpr int PS_CTAS = 6;                         // per SM (80 registers; 5 and 8 within 3%)
 constexpr int PS_WARPS = PS_THREADS / 32;
 constexpr int PS_VIRT = PT_THREADS / PS_THREADS;   // the plain search's threads per thread
 constexpr int PS_CELLS = 121;
@@ -696,9 +696,10 @@ __device__ __forceinline__ void list_add(bool hit, short v, short *list, int *to
 // The plain FP64 evaluation of n listed candidates, a thread each (no list:
 // every candidate, of a pixel out of the screen's range): this thread's best
 // value and its index.
-__device__ __noinline__ void plain_candidates(const short *list, int n, double2 f, double step, const PixelConsts &pc,
-                                              bool ring, double kmean, double rescale, double dn,
-                                              int npop, const double *re, const double *im,
+__device__ __noinline__ void plain_candidates(const short *list, int n, double2 f,
+                                              double step, const PixelConsts &pc, bool ring,
+                                              double kmean, double rescale, double dn, int npop,
+                                              const double *re, const double *im,
                                               const short *idx, const int *__restrict__ hrow,
                                               double &best, int &bidx) {
     for (int i = threadIdx.x; i < n; i += PS_THREADS) {

@@ -166,8 +166,9 @@ k_merge_scatter(const int *__restrict__ pd, const int *__restrict__ pr,
 // the GPU: the warps of a CTA would meet in the same pixels of one state.
 // The reductions in L2 bound both.  848,000 pairs of 1,003 frames over 4,500
 // rows of 185^2 take 1.88 ms, both kernels (1.95 with every row here, 2.56 with
-// one CTA per SM, 3.75 with every photon turned); 101,000 pairs of 1,138 frames over 4,400 rows of 174^2,
-// three of them dense, 0.73 ms by the scatter and 1.07 by row.
+// one CTA per SM, 3.75 with every photon turned); 101,000 pairs of 1,138
+// frames over 4,400 rows of 174^2, three of them dense, 0.73 ms by the scatter
+// and 1.07 by row.
 constexpr int MR_THREADS = 1024;
 constexpr int MR_DENSE = 2;
 constexpr int MR_MIN_PAIRS = 16;   // a row's pairs before its photons are counted
@@ -193,97 +194,98 @@ k_merge_rows(const int *__restrict__ pd, const double *__restrict__ pll,
     double *view = images + (long long)blockIdx.x * npix;
     // the CTA's rows r = blockIdx.x + k gridDim.x, tested MR_THREADS at a time
     for (long long base = blockIdx.x; base < n_rows; base += (long long)gridDim.x * MR_THREADS) {
-    __syncthreads();   // the previous list's readers are done
-    if (threadIdx.x == 0) n_list = 0;
-    __syncthreads();
-    const long long rt = base + (long long)threadIdx.x * gridDim.x;
-    if (rt < n_rows) {
-        row_done[rt] = 0;
-        if (row_off[rt + 1] - row_off[rt] >= MR_MIN_PAIRS) list[atomicAdd(&n_list, 1)] = (int)rt;
-    }
-    __syncthreads();
-    for (int kr = 0; kr < n_list; ++kr) {
-        const long long r = list[kr];
-        const long long a = row_off[r], b = row_off[r + 1];
-        const long long s0 = r / num_rot, j = r - s0 * num_rot;
-        const double ac = rot_cs[2 * j], as = rot_cs[2 * j + 1];
-        double *acc = num + s0 * npix;
-        __syncthreads();   // the previous row's readers are done
-        if (threadIdx.x == 0) n_phot = 0;
+        __syncthreads();   // the previous list's readers are done
+        if (threadIdx.x == 0) n_list = 0;
         __syncthreads();
-        // the row's weight and photon entries
-        double wp = 0.;
-        unsigned np = 0;
-        for (long long i = a + threadIdx.x; i < b; i += MR_THREADS) {
-            const int pair = row_cand[i], d = pd[pair];
-            const double p = exp(pll[pair] - logz[d]);
-            if (!(p >= p_min)) continue;
-            wp += p * scales[d];
-            np += (unsigned)(ones[d] + multi[d]);
-        }
-        wp = warp_sum(wp);
-        np = __reduce_add_sync(RSPI_FULL_MASK, np);
-        if (lane == 0) {
-            wsum[wid] = wp;
-            if (np) atomicAdd(&n_phot, (unsigned long long)np);
+        const long long rt = base + (long long)threadIdx.x * gridDim.x;
+        if (rt < n_rows) {
+            row_done[rt] = 0;
+            if (row_off[rt + 1] - row_off[rt] >= MR_MIN_PAIRS)
+                list[atomicAdd(&n_list, 1)] = (int)rt;
         }
         __syncthreads();
-        if (n_phot * MR_DENSE < (unsigned long long)npix) continue;
-        if (threadIdx.x == 0) {
-            double t = 0.;
-            for (int k = 0; k < MR_THREADS / 32; ++k) t += wsum[k];
-            w[r] = t;
-            row_done[r] = 1;
-        }
-        for (int t = threadIdx.x; t < npix; t += MR_THREADS) __stcg(view + t, 0.);
-        __threadfence();
-        // a thread tests a pair (most of a row's may be below p_min); the warps
-        // share those that are not, several to a pair when they are few
-        for (long long i0 = a; i0 < b; i0 += MR_THREADS) {
-            __syncthreads();   // the previous batch's readers are done
-            if (threadIdx.x == 0) n_sig = 0;
+        for (int kr = 0; kr < n_list; ++kr) {
+            const long long r = list[kr];
+            const long long a = row_off[r], b = row_off[r + 1];
+            const long long s0 = r / num_rot, j = r - s0 * num_rot;
+            const double ac = rot_cs[2 * j], as = rot_cs[2 * j + 1];
+            double *acc = num + s0 * npix;
+            __syncthreads();   // the previous row's readers are done
+            if (threadIdx.x == 0) n_phot = 0;
             __syncthreads();
-            if (i0 + threadIdx.x < b) {
-                const int pair = row_cand[i0 + threadIdx.x], d = pd[pair];
+            // the row's weight and photon entries
+            double wp = 0.;
+            unsigned np = 0;
+            for (long long i = a + threadIdx.x; i < b; i += MR_THREADS) {
+                const int pair = row_cand[i], d = pd[pair];
                 const double p = exp(pll[pair] - logz[d]);
-                if (p >= p_min) {
-                    const int k = atomicAdd(&n_sig, 1);
-                    sig_d[k] = d;
-                    sig_p[k] = p;
-                }
+                if (!(p >= p_min)) continue;
+                wp += p * scales[d];
+                np += (unsigned)(ones[d] + multi[d]);
+            }
+            wp = warp_sum(wp);
+            np = __reduce_add_sync(RSPI_FULL_MASK, np);
+            if (lane == 0) {
+                wsum[wid] = wp;
+                if (np) atomicAdd(&n_phot, (unsigned long long)np);
             }
             __syncthreads();
-            const int share = n_sig > 0 ? max(1, MR_THREADS / 32 / n_sig) : 1;
-            for (int q = wid / share; q < n_sig; q += MR_THREADS / 32 / share) {
-                const int d = sig_d[q];
-                const double p = sig_p[q];
-                const int n_o = ones[d], n_m = multi[d];
-                const long long oa = ones_accum[d], ma = multi_accum[d];
-                for (int k = lane + 32 * (wid % share); k < n_o + n_m; k += 32 * share) {
-                    int pix;
-                    double cnt;
-                    if (k < n_o) {
-                        pix = place_ones[oa + k];
-                        cnt = 1.;
-                    } else {
-                        pix = place_multi[ma + k - n_o];
-                        cnt = (double)count_multi[ma + k - n_o];
+            if (n_phot * MR_DENSE < (unsigned long long)npix) continue;
+            if (threadIdx.x == 0) {
+                double t = 0.;
+                for (int k = 0; k < MR_THREADS / 32; ++k) t += wsum[k];
+                w[r] = t;
+                row_done[r] = 1;
+            }
+            for (int t = threadIdx.x; t < npix; t += MR_THREADS) __stcg(view + t, 0.);
+            __threadfence();
+            // a thread tests a pair (most of a row's may be below p_min); the
+            // warps share those that are not, several to a pair when they are few
+            for (long long i0 = a; i0 < b; i0 += MR_THREADS) {
+                __syncthreads();   // the previous batch's readers are done
+                if (threadIdx.x == 0) n_sig = 0;
+                __syncthreads();
+                if (i0 + threadIdx.x < b) {
+                    const int pair = row_cand[i0 + threadIdx.x], d = pd[pair];
+                    const double p = exp(pll[pair] - logz[d]);
+                    if (p >= p_min) {
+                        const int k = atomicAdd(&n_sig, 1);
+                        sig_d[k] = d;
+                        sig_p[k] = p;
                     }
-                    if (pix >= 0 && pix < npix) atomicAdd(view + pix, p * cnt);
+                }
+                __syncthreads();
+                const int share = n_sig > 0 ? max(1, MR_THREADS / 32 / n_sig) : 1;
+                for (int q = wid / share; q < n_sig; q += MR_THREADS / 32 / share) {
+                    const int d = sig_d[q];
+                    const double p = sig_p[q];
+                    const int n_o = ones[d], n_m = multi[d];
+                    const long long oa = ones_accum[d], ma = multi_accum[d];
+                    for (int k = lane + 32 * (wid % share); k < n_o + n_m; k += 32 * share) {
+                        int pix;
+                        double cnt;
+                        if (k < n_o) {
+                            pix = place_ones[oa + k];
+                            cnt = 1.;
+                        } else {
+                            pix = place_multi[ma + k - n_o];
+                            cnt = (double)count_multi[ma + k - n_o];
+                        }
+                        if (pix >= 0 && pix < npix) atomicAdd(view + pix, p * cnt);
+                    }
                 }
             }
+            __threadfence();
+            __syncthreads();   // the image is complete (in L2)
+            for (int t = threadIdx.x; t < npix; t += MR_THREADS) {
+                const double v = __ldcg(view + t);
+                if (v == 0.) continue;
+                int ix, iy;
+                double fx, fy;
+                if (footprint(t / size, t % size, size, ac, as, ix, iy, fx, fy))
+                    scatter4(acc, size, ix, iy, fx, fy, v);
+            }
         }
-        __threadfence();
-        __syncthreads();   // the image is complete (in L2)
-        for (int t = threadIdx.x; t < npix; t += MR_THREADS) {
-            const double v = __ldcg(view + t);
-            if (v == 0.) continue;
-            int ix, iy;
-            double fx, fy;
-            if (footprint(t / size, t % size, size, ac, as, ix, iy, fx, fy))
-                scatter4(acc, size, ix, iy, fx, fy, v);
-        }
-    }
     }
 }
 
@@ -384,9 +386,10 @@ extern "C" int rspi_merge_rows(const int *pair_d, const int *pair_r, const doubl
                                long long size, const double *cov, double *num, double *den,
                                double *w, double *intens, int *row_done, double *images,
                                long long n_images, cudaStream_t stream) {
-    if (!pair_d || !pair_r || !pair_ll || !row_off || !row_cand || !logz || !scales || !ones || !multi ||
-        !ones_accum || !multi_accum || !rot_cs || !cov || !num || !den || !w || !intens ||
-        !row_done || !images || n_images < 1 || n_states0 <= 0 || num_rot <= 0 || size <= 1 || size > 46340)
+    if (!pair_d || !pair_r || !pair_ll || !row_off || !row_cand || !logz || !scales || !ones ||
+        !multi || !ones_accum || !multi_accum || !rot_cs || !cov || !num || !den || !w ||
+        !intens || !row_done || !images || n_images < 1 || n_states0 <= 0 || num_rot <= 0 ||
+        size <= 1 || size > 46340)
         return RSPI_ERR_ARG;
     const long long npix = size * size, n_rows = n_states0 * num_rot;
     cudaMemsetAsync(num, 0, sizeof(double) * n_states0 * npix, stream);

@@ -188,7 +188,9 @@ k_nll_dense_grid(const double *__restrict__ fre, const double *__restrict__ fim,
                                ((double)(z2 * z2 + w2 * w2) + (double)(z3 * z3 + w3 * w3));
                     } else {
                         // the values are widened for the gradients anyway
-                        auto sq = [](double r, double i, double t) { return fma(r, r, fma(i, i, t)); };
+                        auto sq = [](double r, double i, double t) {
+                            return fma(r, r, fma(i, i, t));
+                        };
                         a64 = sq(z0, w0, sq(z1, w1, sq(z2, w2, sq(z3, w3, a64))));
                         gr[k][0] = fma(s2, (double)z0, gr[k][0]);
                         gi[k][0] = fma(s2, (double)w0, gi[k][0]);
@@ -205,7 +207,8 @@ k_nll_dense_grid(const double *__restrict__ fre, const double *__restrict__ fim,
                         const double q0 = (double)h0, q1 = (double)h1;
                         d64 = fma((double)a.y, fma(ap, p0, bp * p1) + fma(aq, q0, bq * q1), d64);
                         const double ff = (double)a.x;
-                        const double cp = ff * fma(bp, p0, -ap * p1), cq = ff * fma(bq, q0, -aq * q1);
+                        const double cp = ff * fma(bp, p0, -ap * p1);
+                        const double cq = ff * fma(bq, q0, -aq * q1);
                         x64 = fma((double)x, cp, fma(-(double)y, cq, x64));
                         y64 = fma((double)y, cp, fma((double)x, cq, y64));
                     }
@@ -265,7 +268,8 @@ struct GridTables {
 
 int dense_grid_tile(int precision, long long size) {
     // a detector whose phase tables alone leave no room for the radii's
-    if (size <= 1 || (precision == 1 ? 16LL : 8LL) * DG_FRAMES * (size + 2) > DG_SMEM / 2) return -1;
+    if (size <= 1 || (precision == 1 ? 16LL : 8LL) * DG_FRAMES * (size + 2) > DG_SMEM / 2)
+        return -1;
     return precision == 0 ? DG_THREADS * DG_ORBITS<float>
                           : precision == 1 ? DG_THREADS * DG_ORBITS<double> : -1;
 }
@@ -303,9 +307,9 @@ int launch_dense_grid(const GridTables &g, long long n_pix, int size, const doub
     long long per = ((n_frames + want - 1) / want + DG_FRAMES - 1) / DG_FRAMES * DG_FRAMES;
     const dim3 grid((unsigned)tiles, (unsigned)((n_frames + per - 1) / per));
     k_nll_dense_grid<CT, GRAD><<<grid, DG_THREADS, smem, stream>>>(
-        fre, fim, fstride, v, bg_sum, size, reinterpret_cast<const int4 *>(g.order), g.xy, g.rad_id, g.rad_q,
-        g.tile_rads, (int)n_orb, dia, sx, sy,
-        scale, n_frames, per, zero_dia, out, gfre, gfim, gdia, gsx, gsy, gscale);
+        fre, fim, fstride, v, bg_sum, size, reinterpret_cast<const int4 *>(g.order), g.xy,
+        g.rad_id, g.rad_q, g.tile_rads, (int)n_orb, dia, sx, sy, scale, n_frames, per, zero_dia,
+        out, gfre, gfim, gdia, gsx, gsy, gscale);
     return RSPI_OK;
 }
 

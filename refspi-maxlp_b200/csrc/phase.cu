@@ -40,6 +40,7 @@ constexpr int MAX_RADIUS = 64;       // longest Gaussian half-width
 constexpr int DFT_THREADS = 256;
 constexpr int DFT_SPLIT = 2;         // threads per output pair
 constexpr int DFT_LINES = 2;         // lines per CTA: they share the table reads
+static_assert(DFT_SPLIT >= DFT_LINES, "a thread of an output pair finishes each line");
 
 // Shared memory of a CTA: the table, and per line its values and results.
 __device__ __forceinline__ double2 *dft_lines(double2 *smem, int n, int which) {

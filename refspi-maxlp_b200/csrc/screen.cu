@@ -2,8 +2,8 @@
 //
 // 1. FP32 screening pass (ll_sets.cu, ll_quad4.cu, ll_stream.cu): rotated
 //    log-slices stored in FP32, photons as 16-bit sel indices with counts
-//    expanded (a pixel with k photons is k entries, built here).  Sums are
-//    FP32.
+//    expanded (a pixel with k photons is k entries, built here) or, in the
+//    frame sets, entries of up to eight photons.  Sums are FP32.
 // 2. Per frame, every state whose screened value is within
 //    delta + 2 * eps_d of the frame's screened maximum becomes a candidate,
 //    where eps_d bounds |LL32 - LL64| (storage rounding of the slices,
@@ -11,7 +11,9 @@
 //    carries posterior mass above exp(-delta) is a candidate.
 // 3. Candidates are rescored in FP64 with the same slice function, packed
 //    entries and summation order as the FP64 form, so rmax, the maximum and
-//    the log-sum-exp equal the FP64 form's values.
+//    the log-sum-exp equal the FP64 form's values.  Dense frames that fill
+//    most likelihood columns are rescored over the columns
+//    (k_rescore_dense): the same FP64 terms in another order.
 #include <cooperative_groups.h>
 
 #include "rspi_common.cuh"

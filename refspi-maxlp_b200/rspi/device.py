@@ -656,7 +656,8 @@ class EStep:
              s)
         self.ph.err.check('frame-set entries')
         bad = torch.zeros(1, dtype=_i32, device=dev)
-        call('rspi_sets_entries_check' + form, ptr(entries), max(1, total) * 128, part_w, ptr(bad), s)
+        call('rspi_sets_entries_check' + form, ptr(entries), max(1, total) * 128, part_w, ptr(bad),
+             s)
         if int(bad.item()) != 0:
             raise RuntimeError('%d frame-set entries outside the staged part' % int(bad.item()))
         # each frame's FP32 summation length for the candidate threshold:
@@ -1019,8 +1020,8 @@ class Merge:
         else:
             # the rescoring left the candidates grouped by likelihood row
             call('rspi_merge_rows', ptr(es.cand_d), ptr(es.cand_r), ptr(es.cand_ll),
-                 ptr(es.row_cand_off), ptr(es.row_cand), ptr(es.logz), self.p_min, ptr(ph.scales), ptr(ph.ones),
-                 ptr(ph.multi), ptr(ph.ones_accum), ptr(ph.multi_accum), ptr(ph.place_ones),
+                 ptr(es.row_cand_off), ptr(es.row_cand), ptr(es.logz), self.p_min,
+                 ptr(ph.scales), ptr(ph.ones), ptr(ph.multi), ptr(ph.ones_accum), ptr(ph.multi_accum), ptr(ph.place_ones),
                  ptr(ph.place_multi), ptr(ph.count_multi), es.n_states0, es.num_rot,
                  ptr(es.rot_cs), es.size, ptr(self.cov), ptr(self.num), ptr(self.den),
                  ptr(self.w), ptr(self.intens), ptr(self.row_done), ptr(self.images),
@@ -1129,11 +1130,14 @@ class MStep:
         if num_rot <= PIXEL_MAP_MAX_ROT and n_map <= min(PIXEL_MAP_MAX, n_list):
             # a table of the rotations' pixel maps, built once per rotation
             # table (the EMC's fixed angles), where the photon lists read its
-            # entries at least once each.  Below that the search per photon
-            # costs less: 10 us against 20 us at 1,000 frames of 500 photons
-            # (180 rotations of 101^2), and no 10 M-entry table for a phaser
-            # whose frames all have their own angle; above it the table wins
-            # (0.25 ms against 0.9 ms at 20,000 frames of 2,000 photons, 185^2)
+            # entries at least once each: 0.28 ms against 0.36 a call at
+            # 20,000 frames of 2,000 photons (180 rotations of 185^2).  Below
+            # that the table saves little a call and takes some ten of them to
+            # pay for itself: 0.067 against 0.103 ms, 0.2 ms to build and 0.85
+            # for its first memory, at 1,000 frames of 2,000 photons; 0.034
+            # against 0.047, 0.1 to build, at 1,000 of 500 on 101^2.  A phaser
+            # whose frames all have their own angle would build 10 M entries
+            # in every call.
             off, rows = self.pixel_map(rot_cs)
             call('rspi_maxlp_histogram_map', ptr(ph.ones), ptr(ph.multi), ptr(ph.ones_accum),
                  ptr(ph.multi_accum), ptr(ph.place_ones), ptr(ph.place_multi),

@@ -147,25 +147,27 @@ KERNELS_PER_CALL = {
     'rspi_photon_offsets': 4, 'rspi_powder': 2, 'rspi_ll_entry_rows': 1, 'rspi_scan_rows': 1,
     'rspi_ll_entry_fill': 1, 'rspi_holo_slices': 2, 'rspi_vscale_init': 1,
     'rspi_rot_log_slices': 1, 'rspi_holo_pairs': 1, 'rspi_rot_log_slices_pairs': 1,
-    'rspi_loglike': 1, 'rspi_frame_reduce': 1,
-    'rspi_maxlp_frame_params': 1, 'rspi_maxlp_histogram': 1, 'rspi_maxlp_pixel_map': 3,
-    'rspi_maxlp_histogram_map': 1, 'rspi_maxlp_pattern': 1,
-    'rspi_maxlp_pattern_screened': 1, 'rspi_log2_error_max': 1,
+    'rspi_loglike': 1, 'rspi_frame_reduce': 1, 'rspi_maxlp_frame_params': 1,
+    'rspi_maxlp_histogram': 1, 'rspi_maxlp_pixel_map': 3, 'rspi_maxlp_histogram_map': 1,
+    'rspi_maxlp_pattern': 1, 'rspi_maxlp_pattern_screened': 1, 'rspi_log2_error_max': 1,
     'rspi_maxlp_pixel_frames': 1, 'rspi_maxlp_pixel_values': 1, 'rspi_maxlp_fcalc': 1,
     'rspi_sphere_ramp': 1, 'rspi_quad4_entry_groups': 1, 'rspi_quad4_entry_fill': 2,
-    'rspi_screen_loglike7': 1, 'rspi_quad4_part_sums_floats': 0,
-    'rspi_mean': 1, 'rspi_ll16_entry_rows': 1, 'rspi_ll16_entry_fill': 1, 'rspi_screen_candidates': 3, 'rspi_rescore': 5, 'rspi_rescore_dense': 4,
-    'rspi_loglike_stream': 1, 'rspi_posterior_pairs': 3,
-    'rspi_entries16_check': 1, 'rspi_emc_nll': 2, 'rspi_emc_nll_grid': 2, 'rspi_cdft2': 2, 'rspi_phase_support': 5,
-    'rspi_phase_proj_fourier': 1, 'rspi_phase_proj_real': 3, 'rspi_sets_counts': 1, 'rspi_sets_group': 1, 'rspi_sets_steps': 1,
-    'rspi_sets_fill': 1, 'rspi_sets_counts32': 1, 'rspi_sets_fill32': 1, 'rspi_sets_entries_check32': 1,
-    'rspi_screen_loglike_items': 1,
+    'rspi_screen_loglike7': 1, 'rspi_quad4_part_sums_floats': 0, 'rspi_mean': 1,
+    'rspi_ll16_entry_rows': 1, 'rspi_ll16_entry_fill': 1, 'rspi_screen_candidates': 3,
+    'rspi_rescore': 5, 'rspi_rescore_dense': 4, 'rspi_loglike_stream': 1,
+    'rspi_posterior_pairs': 3, 'rspi_entries16_check': 1, 'rspi_emc_nll': 2,
+    'rspi_emc_nll_grid': 2, 'rspi_cdft2': 2, 'rspi_phase_support': 5,
+    'rspi_phase_proj_fourier': 1, 'rspi_phase_proj_real': 3, 'rspi_sets_counts': 1,
+    'rspi_sets_group': 1, 'rspi_sets_steps': 1, 'rspi_sets_fill': 1, 'rspi_sets_counts32': 1,
+    'rspi_sets_fill32': 1, 'rspi_sets_entries_check32': 1, 'rspi_screen_loglike_items': 1,
     'rspi_rot_log_slices_sets': 1, 'rspi_holo_quads32': 1, 'rspi_sets_part_sums_floats': 0,
     'rspi_screen_loglike_sets': 1, 'rspi_frame_max_finalize': 1,
-    'rspi_screen_candidates_cols': 4, 'rspi_rescore_cols': 5, 'rspi_nll': 2, 'rspi_nll_grid': 2, 'rspi_screen_candidates_noalloc': 3, 'rspi_merge_coverage': 1, 'rspi_merge': 2, 'rspi_merge_rows': 3,
-    'rspi_dense_frames': 1, 'rspi_rot_log_split': 1, 'rspi_dense_loglike': 1,
-    'rspi_maxlp_grid': 2, 'rspi_dense_frames_u8': 1, 'rspi_rot_log_fixed': 1, 'rspi_rot_log_fixed_pairs': 1,
-    'rspi_dense_loglike_i8': 1, 'rspi_sets_entries_check': 1, 'rspi_sim_views': 1, 'rspi_sim_counts': 1,
+    'rspi_screen_candidates_cols': 4, 'rspi_rescore_cols': 5, 'rspi_nll': 2, 'rspi_nll_grid': 2,
+    'rspi_screen_candidates_noalloc': 3, 'rspi_merge_coverage': 1, 'rspi_merge': 2,
+    'rspi_merge_rows': 3, 'rspi_dense_frames': 1, 'rspi_rot_log_split': 1,
+    'rspi_dense_loglike': 1, 'rspi_maxlp_grid': 2, 'rspi_dense_frames_u8': 1,
+    'rspi_rot_log_fixed': 1, 'rspi_rot_log_fixed_pairs': 1, 'rspi_dense_loglike_i8': 1,
+    'rspi_sets_entries_check': 1, 'rspi_sim_views': 1, 'rspi_sim_counts': 1,
     'rspi_sim_poisson': 1, 'rspi_sim_sparse_counts': 1, 'rspi_sim_sparse_fill': 1,
 }
 # counts scanned by an entry point, from its arguments; its scan's launches
