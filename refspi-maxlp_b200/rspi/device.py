@@ -293,6 +293,7 @@ class EStep:
         if entries not in ('auto', 'single'):
             raise ValueError('entries must be auto or single')
         self.count_entries = entries == 'auto'
+        self.counts_pay = None   # not known yet
         if kernel is None:   # default likelihood kernel of each form
             kernel = 'sets' if form == 'screen' else 'stream'
         kernels = {'fp64': ('stream', 'dynamic'), 'screen': ('stream', 'quad4', 'sets'),
@@ -613,13 +614,17 @@ class EStep:
         pz = self.p_row - 32
         parts, part_w = self._quad4_parts()
         counts = torch.empty(n * 32, dtype=_i32, device=dev)
-        counted = self.count_entries and part_w <= SETS_COUNTED_COLS
+        # whether counts pay does not depend on the parts: asked once
+        counted = self.count_entries and self.counts_pay is not False and \
+            part_w <= SETS_COUNTED_COLS
         if counted:
             call('rspi_sets_counts32', ptr(ll['entries']), ptr(ll['row_off']), n, pz, parts,
                  part_w, ptr(counts), s)
             tot = counts.view(n, 32).sum(1)
-            phot = int(ll['frame_sel_photons'].sum())
-            counted = COUNT_GAIN * (phot - int(tot.sum())) >= phot
+            if self.counts_pay is None:
+                phot = int(ll['frame_sel_photons'].sum())
+                self.counts_pay = COUNT_GAIN * (phot - int(tot.sum())) >= phot
+            counted = self.counts_pay
         if not counted:
             ll = self.ll16
             call('rspi_sets_counts', ptr(ll['entries']), ptr(ll['row_off']), n, pz, parts, part_w,

@@ -45,3 +45,27 @@ def test_a_configuration_that_names_the_kernel_keeps_its_layout(extra, tmp_path)
     rec = EMC(write_case(str(tmp_path), data=data, size=size, num_rot=3, shiftx='0 1 2',
                          shifty='0 0 1', sphere_dia='6 8 2', need_scaling=True, extra=extra))
     assert rec.estep.kernel == 'sets' and rec.estep.wide['counted']
+
+
+@pytest.mark.parametrize('mean,pays', [(0.02, False), (1.5, True)])
+def test_whether_counts_pay_is_asked_once(mean, pays, monkeypatch):
+    """Another tiling (the tuner tries several) rebuilds the entries without
+    counting them in both layouts again where the first count rejected one."""
+    from rspi import device
+    from rspi.photonfile import sparse_from_dense
+    from test_gpu_estep import _estep, _photons
+    size, n = 31, 70
+    d = sparse_from_dense(np.random.default_rng(6).poisson(mean, (n, size * size)))
+    ds = E.parse_photons(d['ones'], d['multi'], d['place_ones'], d['place_multi'],
+                         d['count_multi'], size * size, True)
+    sx, sy, dia, _ = E.generate_states((0., 1., 2), (0., 0., 1), (6., 8., 2))
+    es = _estep(_photons(ds, False), size, 3, sx, sy, dia, ds['bg'], form='screen',
+                states_per_tile=4)
+    assert es.wide['counted'] == pays
+    seen = []
+    call = device.call
+    monkeypatch.setattr(device, 'call', lambda name, *a: (seen.append(name), call(name, *a))[1])
+    es.configure(screen_parts=2)
+    assert es.wide['counted'] == pays and es.wide['n_parts'] == 2
+    assert ('rspi_sets_counts32' in seen) == pays
+    assert ('rspi_sets_counts' in seen) == (not pays)
