@@ -472,7 +472,8 @@ int rspi_rescore(const int *cand_d, const int *cand_r, const long long *cand_off
 /* rspi_rescore for densely stored frames (n_data x size^2 counts): each row's
  * FP64 rotated slice is built a tile of columns at a time and multiplied with
  * its candidates' counts there, instead of walking their sparse entries (the
- * sums differ from rspi_rescore's by their FP64 rounding). */
+ * sums differ from rspi_rescore's by their FP64 rounding).  For frames whose
+ * photons fill most likelihood columns; a candidate costs all n_sel columns. */
 int rspi_rescore_dense(const int *cand_d, const int *cand_r, const long long *cand_off,
                        long long n_data, long long capacity, long long n_rows,
                        const unsigned short *frames, const double *holo, long long num_rot,
@@ -537,8 +538,8 @@ int rspi_merge(const int *pair_d, const int *pair_r, const double *pair_ll,
  * the candidates: row r's pairs are row_cand[row_off[r] .. row_off[r + 1]),
  * pair_r their rows, row_off[n_rows] their number; row_done: n_rows ints of
  * scratch.
- * `images` holds n_images scratch images of size^2 doubles, one per CTA (two
- * per SM).  Sums differ from rspi_merge's by their FP64 rounding. */
+ * `images` holds n_images >= 1 scratch images of size^2 doubles, one per CTA
+ * (two per SM are fastest).  Sums differ from rspi_merge's by their FP64 rounding. */
 int rspi_merge_rows(const int *pair_d, const int *pair_r, const double *pair_ll,
                     const long long *row_off, const int *row_cand, const double *logz,
                     double p_min, const double *scales, const int *ones, const int *multi,

@@ -435,10 +435,9 @@ __global__ void k_dense_frames_u8(const unsigned short *__restrict__ frames, lon
 // GPU too), a warp 128 columns, 32 neighbours at a time: the columns' rotated
 // positions depend on (j, column) only and are computed once for the states,
 // and the four digits of four lanes' columns change places (two shuffles) for
-// one 32-bit store per digit plane.  PAIRS: holo as (w[p], w[p + 1]) pairs, so that a
-// corner row is one 16-byte load.  Bound by L1 (75% of its wavefronts with
-// four columns of a thread side by side and 8-byte loads) and by issue; 9,720
-// rows x 47,616 columns: 3.25 ms with a row per CTA, 2.99 with eight states,
+// one 32-bit store per digit plane.  PAIRS: holo as (w[p], w[p + 1]) pairs, so
+// that a corner row is one 16-byte load.  Bound by L1 (77%) and issue (76%);
+// 9,720 rows x 47,616 columns: 3.25 ms with a row per CTA, 2.99 with eight states,
 // 2.87 with neighbouring columns, 2.67 with pairs and four CTAs per SM (three
 // 2.85, five 2.92; four states 2.81, sixteen 2.99), 2.50 in parts (RQ_CTAS 16
 // 2.66, 32 2.52, 128 2.53).  108 rows of 4 rotations: 0.14 ms with a row per

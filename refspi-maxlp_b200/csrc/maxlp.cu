@@ -598,8 +598,10 @@ k_pattern(double2 *__restrict__ fconv, const int *__restrict__ pixels,
 // candidates' rounded positions (d >= 2^-30 A is required), and the FP64
 // rounding of any candidate of the cell, 2^-30 of the value's terms.
 //
-// What bounds it is instruction issue and, for few pixels, the chain of an
-// iteration: ~14 instructions per (cell, state) for 121 cells instead of ~9
+// What bounds it is instruction fetch (its code does not stay in the SM's
+// instruction cache: the second level serves requests at 99% of its peak, and
+// issue is 44%) and, for few pixels, the chain of an iteration.  It issues a
+// fifth of what the search before it did: ~14 instructions per (cell, state) for 121 cells instead of ~9
 // per (candidate, state) for 1,089, and 4 barriers of four warps instead of
 // 11 of twelve.  Measured, both passes together, against one CTA of 384
 // threads per pixel evaluating every candidate in FP32: 185^2, 20,000 frames

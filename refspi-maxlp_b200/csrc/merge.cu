@@ -164,7 +164,8 @@ k_merge_scatter(const int *__restrict__ pd, const int *__restrict__ pr,
 // pixel) instead of four per photon.  Rows with fewer than npix / MR_DENSE
 // photons are left to k_merge_scatter (row_done 0), which spreads them over
 // the GPU: the warps of a CTA would meet in the same pixels of one state.
-// The reductions in L2 bound both.  848,000 pairs of 1,003 frames over 4,500
+// Both wait for L2: 30 cycles of 33 between a warp's issues, the atomics at 27%
+// of L2's rate.  848,000 pairs of 1,003 frames over 4,500
 // rows of 185^2 take 1.88 ms, both kernels (1.95 with every row here, 2.56 with
 // one CTA per SM, 3.75 with every photon turned); 101,000 pairs of 1,138
 // frames over 4,400 rows of 174^2, three of them dense, 0.73 ms by the scatter

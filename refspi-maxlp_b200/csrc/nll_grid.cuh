@@ -27,7 +27,9 @@ __device__ __forceinline__ void dg_sincos(double x, double *s, double *c) { sinc
 // gradient sums over all of the CTA's frames and the frames' sums over its
 // orbits in FP64, the scale applied once per frame, and the warps transpose
 // the latter as they reduce them: 1.5 instructions per pixel instead of 60.
-// Bound by instruction issue, half of it conversions to FP64 and FP64 adds.
+// Bound by the conversions to FP64 (XU pipe 53% busy) and the orbits' chains at
+// 128 registers (issue 54%).  Opposite pixels' values meet after they are
+// widened, so every term is its pixel's own.
 // Measured, value and gradients, against the kernels that take a sine pair per
 // pixel: 26,836 pixels x 20,000 frames 1.28 ms (4.4), 24,928 x 5,000 0.31 ms
 // (1.17), FP64 with 7,972 x 1,000 0.035 ms (0.10).
