@@ -203,8 +203,10 @@ __device__ __forceinline__ double2 fref_value(double qx, double qy, double qrad,
     const double sval = xmul(xmul(PI, qrad), dia);
     double sn, cs;
     sincos(sval, &sn, &cs);
-    // sval^3 to the last bit or so: the square and the cube with their
-    // rounding errors (pow took a third of the pattern search's set-up)
+    // sval^3 rounded once: the square and the cube with their rounding errors.
+    // pow, 2 to 5% of an iteration, is off by a bit at times; where a pixel's
+    // candidates tie but for rounding (all its frames in one state, a model far
+    // below the reference) the two can choose differently.
     const double s2 = xmul(sval, sval), s3 = xmul(s2, sval);
     const double cube = xadd(s3, fma(fma(sval, sval, -s2), sval, fma(s2, sval, -s3)));
     const double ff = xsub(sn, xmul(sval, cs)) / cube;
